@@ -274,3 +274,60 @@ def tolerance(case):
     if case["kind"] == "write":
         return "exact"
     return {"rel": 7e-3, "max": 1.8e-2, "differ": 0.0}
+
+
+# --------------------------------------------------------------------------------------------------------------- exact
+def _e4m3(b):
+    return b.contiguous().view(torch.float8_e4m3fn).double()
+
+
+def _e2m1(b):
+    """codes, two to a byte (the first in the low nibble), in blocks of sixteen -> (.., blocks, 16)"""
+    table = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64,
+                         device=b.device)
+    codes = torch.stack((b & 15, b >> 4), dim=-1).long()
+    return table[codes].reshape(*b.shape[:-1], b.shape[-1] // 8, 16)
+
+
+def _fp4(slots, D):
+    return (_e2m1(slots[..., :D // 2]) * _e4m3(slots[..., D // 2:])[..., None]).reshape(*slots.shape[:-1], D)
+
+
+def exact(case, seed):
+    """The attention of the step in 64 bits over the bytes that the cache holds once the step's tokens are in it (those
+    bytes have a tolerance of their own, none, and no value here). Decode rows are scaled by the value scale twice, as
+    their entry point's two arguments are, prefill rows once."""
+    if case["kind"] == "write":
+        return None
+    s = prepare(case, seed)
+    s.impl.do_kv_cache_update(s.layer, s.k, s.v, s.cache, s.slots)
+    H, D, G, PS = case["kv_heads"], case["head_dim"], case["group"], case["page"]
+    q_all = s.q.view(-1, H * G, D).double()
+    if case["had"]:
+        signs = torch.randint(0, 2, (D,), generator=torch.Generator().manual_seed(0x6B7634)) * 2 - 1
+        had = torch.ones((1, 1), dtype=torch.float64)
+        while had.shape[0] < D:
+            had = torch.cat((torch.cat((had, had), 1), torch.cat((had, -had), 1)))
+        q_all = (q_all * signs.cuda()) @ (had * D ** -0.5).cuda()
+    out = torch.zeros_like(q_all)
+    qsl, lens, bt = s.meta.query_start_loc.tolist(), s.meta.seq_lens.tolist(), s.meta.block_table
+    for b, L in enumerate(lens):
+        t0, t1 = qsl[b], qsl[b + 1]
+        pages = bt[b, :(L + PS - 1) // PS].long()
+        lim = torch.arange(L - (t1 - t0) + 1, L + 1, device="cuda").repeat_interleave(G)
+        for h in range(H):
+            rows = s.cache[pages, h].reshape(-1, s.cache.shape[3])[:L]
+            if case["k8"]:
+                k, v = _e4m3(rows[:, :D]), _fp4(rows[:, D:], D)
+            else:
+                k, v = _fp4(rows, D), _fp4(s.cache[pages, H + h].reshape(-1, rows.shape[1])[:L], D)
+            qh = q_all[t0:t1, h * G:(h + 1) * G].reshape(-1, D)
+            step = max(1, 2 ** 27 // L)
+            o = []
+            for r in range(0, qh.shape[0], step):
+                w = qh[r:r + step] @ k.T * (D ** -0.5 * GK)
+                w.masked_fill_(torch.arange(L, device="cuda")[None, :] >= lim[r:r + step, None], -math.inf)
+                o.append(torch.softmax(w, dim=1) @ v)
+            out[t0:t1, h * G:(h + 1) * G] = torch.cat(o).view(t1 - t0, G, D) * (GV * GV if t0 < s.n_decode else GV)
+    out = out.view(out.shape[0], H * G * D)
+    return {"decode": out[:s.n_decode], "prefill": out[s.n_decode:], "cache": None}
