@@ -10,6 +10,7 @@ EXPORTS = ("hkv_version", "hkv_error_string", "hkv_last_cuda_error", "hkv_write"
            "hkv_decode", "hkv_combine", "hkv_workspace_status", "hkv_decode_noalloc", "hkv_decode_noalloc_status",
            "hkv_set_option", "hkv_dequant", "hkv_write_rot",
            "hkv_decode_rot", "hkv_write_k8", "hkv_decode_k8", "hkv_dequant_k8",
+           "hkv_prefill", "hkv_prefill_scratch_bytes",
            "hkv_selftest_wait_timeout", "hkv_selftest_codec", "hkv_probe_issue_rates")
 
 _lib = None
@@ -68,6 +69,11 @@ def load():
         L.hkv_dequant_k8.restype = i32
         L.hkv_dequant_k8.argtypes = [vp, vp, vp, C.POINTER(i64), i32, vp, i32, vp, vp, i32, i64, i64, vp, vp, i32, i32,
                                      i32, vp]
+        L.hkv_prefill_scratch_bytes.restype = C.c_size_t
+        L.hkv_prefill_scratch_bytes.argtypes = [C.POINTER(i32), i32, i32, i32, i32, i32, i64, i32]
+        L.hkv_prefill.restype = i32
+        L.hkv_prefill.argtypes = [vp, i32, vp, vp, vp, vp, C.POINTER(i64), i32, vp, i32, i32, C.POINTER(i32), i32, i32, i32,
+                                  i32, i32, f32, f32, i32, vp, i32, i64, vp, C.c_size_t, vp, i32, vp, vp]
         L.hkv_selftest_wait_timeout.restype = i32
         L.hkv_selftest_wait_timeout.argtypes = [vp, i64, vp]
         L.hkv_selftest_codec.restype = i32

@@ -10,10 +10,9 @@
 
 The classes derive from vLLM's base classes when vLLM has already been imported by the process (that is, when vLLM
 loads this plugin); otherwise from small stand-ins, so the surface can be exercised and benchmarked without importing
-vLLM. Rows with more query tokens than the decode threshold (prefill over a cached prefix) take the exact
-dequantisation kernel, chunk by chunk, followed by torch matmuls with a running log-sum-exp (library attention, as the
-reference uses FlashInfer's FA2 and merge_state there, backend.py:517-543); that path is eager and outside the timed
-hot path. There is no fallback to another backend.
+vLLM. Rows with more query tokens than the decode threshold (prompts, chunks of prompts, prompts over a cached prefix)
+take the prefill kernels (the reference uses FlashInfer's FA2 and merge_state there, backend.py:517-543). There is no
+fallback to another backend.
 """
 import os
 import sys
@@ -337,60 +336,33 @@ def _build_classes():
             return output
 
         def _prefill_rows(self, layer, q, v, m, out):
-            """requests with more query tokens than the decode threshold: the request's context (the new tokens were
-            written by do_kv_cache_update) is dequantised exactly in chunks of HORIZON_KVFP4_CHUNK tokens (65,536, the
-            reference's chunk: backend.py:16-25, :519-543) and attended chunk by chunk with a running log-sum-exp, so
-            the memory held per request is bounded by the chunk, not by the context. Causal window of the reference:
-            query token t of ql sees keys j < L - ql + t + 1. Compute dtype fp16 (HORIZON_KVFP4_PF16=1, the reference's
-            default, backend.py:229: code * scale is exact in fp16) or bf16. The global scales are folded into the
-            softmax scale and the output like the reference's sm / vs. Eager torch matmuls (a library path, as the
-            reference calls FlashInfer there), outside the timed decode path."""
-            sm = self.scale * float(layer._k_scale_float)
-            vs = float(layer._v_scale_float)
-            KVH, G, D = self.num_kv_heads, self.G, self.head_size
-            dt = torch.float16 if self.pf16 else torch.bfloat16
-            CH = self.prefill_chunk
-            dev = q.device
-            for row, q0, q1, L in m.prefill_rows:
-                ql = q1 - q0
-                if ql <= 0 or L <= 0:
-                    continue
-                qi = q[q0:q1]
-                if self.had:                                                     # the cached keys are rotated
-                    qi = K.rotate(qi, self._rot(dev)).to(torch.bfloat16)
-                # (KVH, G * ql, D): row g * ql + t of a kv head is query head g, token t
-                qh = qi.view(ql, KVH, G, D).permute(1, 2, 0, 3).reshape(KVH, G * ql, D).to(dt)
-                lim = (L - ql + 1 + torch.arange(ql, device=dev)).repeat(G)      # keys visible to every row
-                n_ch = min(CH, L)
-                kk = torch.empty((n_ch, KVH, D), dtype=dt, device=dev)
-                vv = torch.empty_like(kk)
-                # query rows per block so that one block's scores stay near 256 MB
-                QB = max(1, min(G * ql, (256 << 20) // max(1, KVH * n_ch * 4)))
-                acc = torch.zeros((KVH, G * ql, D), dtype=torch.float32, device=dev)
-                mx = torch.full((KVH, G * ql, 1), float("-inf"), dtype=torch.float32, device=dev)
-                den = torch.zeros((KVH, G * ql, 1), dtype=torch.float32, device=dev)
-                bt_row = m.block_table[row].contiguous()
-                for c0 in range(0, L, CH):
-                    n = min(CH, L - c0)
-                    K.dequant_tokens(v["flat"], v["strides"], v["PS"], bt_row, c0, n, kk, vv, k8=self.k8)
-                    kt = kk[:n].permute(1, 2, 0)                                 # (KVH, D, n)
-                    # (KVH, n, D); the value product always takes fp16 operands: the dequantised values are exact in it
-                    # and the probabilities lie in [0, 1]; both products accumulate and return fp32
-                    vt = vv[:n].permute(1, 0, 2).to(torch.float16)
-                    pos = c0 + torch.arange(n, device=dev)
-                    for r0 in range(0, G * ql, QB):
-                        r1 = min(G * ql, r0 + QB)
-                        s_ = torch.bmm(qh[:, r0:r1], kt, out_dtype=torch.float32) * sm   # (KVH, rows, n), fp32 accumulate and output
-                        s_.masked_fill_(pos[None, None, :] >= lim[None, r0:r1, None], float("-inf"))
-                        nm = torch.maximum(mx[:, r0:r1], s_.amax(dim=-1, keepdim=True))
-                        nm_safe = torch.where(torch.isinf(nm), torch.zeros_like(nm), nm)
-                        p_ = torch.exp(s_ - nm_safe)
-                        al = torch.exp(mx[:, r0:r1] - nm_safe)
-                        den[:, r0:r1] = den[:, r0:r1] * al + p_.sum(dim=-1, keepdim=True)
-                        acc[:, r0:r1] = acc[:, r0:r1] * al + torch.bmm(p_.to(torch.float16), vt, out_dtype=torch.float32)
-                        mx[:, r0:r1] = nm
-                o = acc / den.clamp_min(1e-30) * vs
-                out[q0:q1].copy_(o.view(KVH, G, ql, D).permute(2, 0, 1, 3).reshape(ql, KVH * G, D).to(out.dtype))
+            """requests with more query tokens than the decode threshold, all in one call of the prefill kernels: their
+            contexts (the new tokens were written by do_kv_cache_update) become 16-bit operands in chunks of
+            HORIZON_KVFP4_CHUNK tokens (65,536, the reference's chunk: backend.py:16-25, :519-543), which bounds the
+            memory held. Causal window of the reference: query token t of ql sees keys j < L - ql + t + 1. Compute dtype
+            of the scores fp16 (HORIZON_KVFP4_PF16=1, the reference's default, backend.py:229: code * scale is exact in
+            fp16) or bf16; the value product takes fp16 operands (the dequantised values are exact in it and the
+            probabilities lie in [0, 2^8]); both accumulate in fp32. The global scales are folded into the softmax scale
+            and the output like the reference's sm / vs."""
+            rows = [(row, q0, q1, L) for row, q0, q1, L in m.prefill_rows if q1 > q0 and L > 0]
+            if not rows:
+                return
+            signs = self._rot(q.device)
+            if q.dtype != torch.bfloat16:             # (vLLM passes bf16)
+                if signs is not None:
+                    q, signs = K.rotate(q, signs).to(torch.bfloat16), None
+                q = q.to(torch.float16 if self.pf16 else torch.bfloat16)
+            if q.data_ptr() % 16:
+                q = q.clone()
+            direct = out.is_contiguous() and out.data_ptr() % 16 == 0 and out.dtype in (torch.bfloat16, torch.float32)
+            o = out if direct else torch.empty(out.shape, dtype=torch.float32, device=out.device)
+            bt = m.block_table if m.block_table.is_contiguous() else m.block_table.contiguous()
+            K.prefill(q, v["flat"], v["strides"], v["PS"], bt, rows, self.scale * float(layer._k_scale_float),
+                      float(layer._v_scale_float), self.num_kv_heads, o, chunk=self.prefill_chunk, k_f16=self.pf16,
+                      signs=signs, k8=self.k8, workspace=self._state(q.device)["ws"])
+            if not direct:
+                for _, q0, q1, _ in rows:
+                    out[q0:q1].copy_(o[q0:q1])
 
     return dict(HorizonFp4Backend=HorizonFp4Backend, HorizonFp4Metadata=HorizonFp4Metadata,
                 HorizonFp4Builder=HorizonFp4Builder, HorizonFp4Impl=HorizonFp4Impl)

@@ -1,0 +1,130 @@
+"""The prefill kernels (csrc/hkv_prefill.cu) against attention in fp64 over the same cache bytes, at the sizes where they
+can go wrong: row tiles and key tiles with remainders, groups that do not divide 128, row tiles whose keys are divided
+among CTAs, contexts longer than the chunk, many requests in one call, query tokens without any visible key."""
+import numpy as np
+import pytest
+import torch
+
+import synth
+from cases import bf16_tensor
+from horizon_kernels_b200 import kernels as K
+from horizon_kernels_b200 import layout as Lt
+from oracle import kvfp4 as O
+
+pytestmark = pytest.mark.gpu
+
+
+def run_case(qls, lens, KVH, G, D, PS=16, chunk=65536, k_f16=True, out_dtype=torch.bfloat16, seed=5, qk_scale=None):
+    c = synth.paged_case(seed + D, lens, KVH, G, D, PS, outliers=True, ql_list=qls)
+    dev = torch.device("cuda")
+    gk = torch.full((KVH,), 0.04, device=dev)
+    gv = torch.full((KVH,), 1.0, device=dev)
+    cache = Lt.alloc_cache(c["NP"], PS, KVH, D, device=dev, fill=0x7F)
+    flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
+    K.write(bf16_tensor(c["key"]), bf16_tensor(c["val"]), flat, strides, PS, torch.from_numpy(c["slots"]).to(dev), gk, gv)
+    q = bf16_tensor(c["q"])
+    NT = q.shape[0]
+    out = torch.full((NT + 3, KVH * G, D), 5.0, dtype=out_dtype, device=dev)
+    qsl = [int(x) for x in c["qsl"]]
+    rows = [(b, qsl[b], qsl[b + 1], L) for b, L in enumerate(lens)]
+    sm = D ** -0.5 if qk_scale is None else qk_scale
+    ws = K.alloc_workspace(4, KVH, min(G, 8), D)
+    K.prefill(q, flat, strides, PS, torch.from_numpy(c["bt"]).to(dev), rows, sm * 0.04, 1.0, KVH, out, chunk=chunk,
+              k_f16=k_f16, workspace=ws)
+    assert K.workspace_status(ws) == 0
+    assert (out[NT:] == 5.0).all()
+    lay = O.Layout.slots(PS, KVH, D)
+    ref, _ = O.attention(c["q"], cache.cpu().numpy().reshape(-1), lay, c["bt"], c["seq_lens"], c["qsl"], KVH, sm,
+                         np.full(KVH, 0.04, np.float32), np.ones(KVH, np.float32), 1.0)
+    got, want = out[:NT].float().cpu().numpy().astype(np.float64), np.asarray(ref, np.float64)
+    # probabilities and the output are each rounded to 11 and 8 bits: 2^-9 of a value from the latter, less from the
+    # former; four times the sum of both roundings' root mean squares (1.7e-3)
+    rel = np.linalg.norm(got - want) / max(np.linalg.norm(want), 1e-30)
+    assert rel <= 2.5e-3, rel
+    return out, rows, want
+
+
+SIZES = [
+    ([1], [1]), ([5], [5]), ([128], [128]), ([129], [129]), ([31], [4000]), ([300], [777]), ([64, 33, 2, 257], [64, 1000, 300, 257]),
+]
+
+
+@pytest.mark.parametrize("qls,lens", SIZES)
+@pytest.mark.parametrize("KVH,G,D", [(2, 4, 128), (2, 8, 256)])
+def test_sizes(qls, lens, KVH, G, D):
+    run_case(qls, lens, KVH, G, D)
+
+
+@pytest.mark.parametrize("KVH,G,D,PS", [(1, 1, 128, 16), (3, 6, 128, 32), (1, 12, 256, 64), (4, 6, 256, 16), (1, 64, 128, 16)])
+def test_groups_and_pages(KVH, G, D, PS):
+    run_case([70, 9], [200, 513], KVH, G, D, PS)
+
+
+@pytest.mark.parametrize("chunk", [1, 128, 300, 1024])
+@pytest.mark.parametrize("KVH,G,D", [(2, 4, 128), (1, 8, 256)])
+def test_chunks_keep_a_state(KVH, G, D, chunk):
+    """contexts of several chunks, alone and among requests that share a launch; fp32 output"""
+    run_case([150, 20, 40], [1500, 260, 900], KVH, G, D, chunk=chunk, out_dtype=torch.float32)
+
+
+@pytest.mark.parametrize("D", [128, 256])
+def test_divided_row_tiles(D):
+    """one short request over a long context: every CTA has a part of the same row tiles"""
+    run_case([3], [20000], 1, 4, D)
+
+
+def test_bf16_scores():
+    run_case([100], [500], 2, 4, 128, k_f16=False)
+
+
+@pytest.mark.parametrize("D", [128, 256])
+def test_negative_and_zero_scale(D):
+    run_case([40], [300], 1, 4, D, qk_scale=-0.05)
+    run_case([40], [300], 1, 4, D, qk_scale=0.0)
+
+
+@pytest.mark.parametrize("D", [128, 256])
+def test_tokens_without_keys(D):
+    """more query tokens than context: the first ones see no key and give zeros"""
+    dev = torch.device("cuda")
+    KVH, G, PS, ql, L = 2, 4, 16, 200, 37
+    cache = torch.randint(0, 120, (4, 2 * KVH, PS, Lt.slot_bytes(D)), dtype=torch.uint8, device=dev)
+    flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
+    q = torch.randn(ql, KVH * G, D, device=dev).to(torch.bfloat16)
+    out = torch.full_like(q, 3.0)
+    K.prefill(q, flat, strides, PS, torch.arange(4, dtype=torch.int32, device=dev).view(1, 4), [(0, 0, ql, L)], 1e-3, 1.0,
+              KVH, out)
+    assert (out[:ql - L] == 0).all() and torch.isfinite(out.float()).all() and (out[ql - L:] != 0).any()
+
+
+def test_many_requests():
+    """more requests than one launch takes"""
+    rng = np.random.default_rng(3)
+    qls = [int(x) for x in rng.integers(2, 40, 70)]
+    lens = [q + int(x) for q, x in zip(qls, rng.integers(0, 200, 70))]
+    run_case(qls, lens, 1, 4, 128)
+
+
+def test_graph_capture_and_repeat():
+    """captured once and replayed: the same bits as the eager call"""
+    dev = torch.device("cuda")
+    KVH, G, D, PS, ql, L = 2, 4, 128, 16, 130, 700
+    cache = torch.randint(0, 120, (64, 2 * KVH, PS, Lt.slot_bytes(D)), dtype=torch.uint8, device=dev)
+    flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
+    q = torch.randn(ql, KVH * G, D, device=dev).to(torch.bfloat16)
+    bt = torch.randperm(64, device=dev)[:L // PS + 1].to(torch.int32).view(1, -1)
+    eager, out = torch.zeros_like(q), torch.zeros_like(q)
+    call = lambda o: K.prefill(q, flat, strides, PS, bt, [(0, 0, ql, L)], 1e-3, 1.0, KVH, o)  # noqa: E731
+    call(eager)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(out)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            call(out)
+    torch.cuda.current_stream().wait_stream(side)
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
