@@ -1,10 +1,12 @@
 """ctypes binding of the C ABI in include/hkv.h. There is no fallback: if the CUDA library is missing or does not
 load, every kernel entry point raises."""
 import ctypes as C
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libhkv.so")
+HOST_PATH = os.path.join(HERE, "lib", "hkv_host.so")
 
 EXPORTS = ("hkv_version", "hkv_error_string", "hkv_last_cuda_error", "hkv_write", "hkv_decode_workspace_bytes",
            "hkv_decode", "hkv_combine", "hkv_workspace_status", "hkv_decode_noalloc", "hkv_decode_noalloc_status",
@@ -14,6 +16,7 @@ EXPORTS = ("hkv_version", "hkv_error_string", "hkv_last_cuda_error", "hkv_write"
            "hkv_selftest_wait_timeout", "hkv_selftest_codec", "hkv_probe_issue_rates")
 
 _lib = None
+_host = None
 
 
 class HkvError(RuntimeError):
@@ -86,6 +89,23 @@ def load():
         L.hkv_workspace_status.argtypes = [vp, C.POINTER(i32), vp]
         _lib = L
     return _lib
+
+
+def host():
+    """the native side of the host wrappers (csrc/hkv_host.cpp), bound to the loaded library"""
+    global _host
+    if _host is None:
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m horizon_kernels_b200.build`")
+        L = load()
+        spec = importlib.util.spec_from_file_location("hkv_host", HOST_PATH)
+        h = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(h)
+        h.bind(*[C.cast(f, C.c_void_p).value for f in (
+            L.hkv_write, L.hkv_write_rot, L.hkv_write_k8, L.hkv_decode, L.hkv_decode_rot, L.hkv_decode_k8,
+            L.hkv_prefill_scratch_bytes, L.hkv_prefill)])
+        _host = h
+    return _host
 
 
 def check(code: int, where: str):

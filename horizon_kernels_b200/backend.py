@@ -249,7 +249,7 @@ def _build_classes():
         def _state(self, device):
             """one zeroed decode workspace per device, allocated on first use outside graph capture
             (reference backend.py:263-277)"""
-            key = (str(device), self.num_kv_heads, self.G, self.head_size, self.qlmax)
+            key = (device, self.num_kv_heads, self.G, self.head_size, self.qlmax)
             st = _STATE.get(key)
             if not _STATE.get("options"):
                 # vLLM writes seq_lens and query_start_loc once per step, before the first layer runs, so the decode

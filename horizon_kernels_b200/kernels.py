@@ -1,8 +1,10 @@
 """Host wrappers of the three CUDA kernels, with the call signatures of the reference's serving module
 (nvidia-sm120/horizon_kvfp4/kernels/kv_fp4_serving.py): `write`, `decode_ragged`, `flat_views`, `plan_splits`.
 
-The wrappers only marshal pointers, sizes and the current CUDA stream into the C ABI (include/hkv.h). They allocate
-nothing and never synchronise, so calls can be captured in a CUDA graph. There is no CPU or PyTorch fallback."""
+The wrappers only marshal pointers, sizes and the current CUDA stream into the C ABI (include/hkv.h): natively
+(csrc/hkv_host.cpp) for arguments of the plain form, in Python for the rest, which is also where wrong arguments raise.
+They never synchronise and allocate nothing (prefill: its scratch, from torch's allocator), so calls can be captured in
+a CUDA graph. There is no CPU or PyTorch fallback."""
 import ctypes as C
 
 import torch
@@ -100,6 +102,12 @@ def write(key, value, flat, strides, PS, slot_mapping, gk, gv, search=True, sign
     signs (D,) fp32 of +-1 on the device: the keys are rotated (FWHT(k * signs) * D^-0.5 in fp32) before they are
     quantised. Bit-exact to the reference's write_reference (kv_fp4_ref.py:233-245). Signature of
     kv_fp4_serving.py:994."""
+    rc = (_lib._host or _lib.host()).write(key, value, flat, strides, PS, slot_mapping, gk, gv, search, signs, k8)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "hkv_write")
+        return
+    # not the plain form that the native side takes: check, raise or serve it here
     if k8 and signs is not None:
         raise ValueError("the K8V4 slot keeps FP8 keys: no rotation")
     if key.dtype != torch.bfloat16 or value.dtype != torch.bfloat16:
@@ -142,6 +150,12 @@ def decode_ragged(query, flat, strides, PS, block_tables, seq_lens, query_start_
     (nst, ncw, min_chunk, tw) are accepted and ignored. signs (D,) fp32 of +-1 on the device: the keys in the cache
     were written rotated, and the kernel rotates the UNROTATED query it is given the same way.
     Signature of kv_fp4_serving.py:894-895."""
+    rc = (_lib._host or _lib.host()).decode(query, flat, strides, PS, block_tables, seq_lens, query_start_loc, bmm1_scale,
+                                            bmm2_scale, gk, gv, qlmax, out, workspace, splits, signs, k8)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "hkv_decode")
+        return out
     if k8 and signs is not None:
         raise ValueError("the K8V4 slot keeps FP8 keys: no rotation")
     if query.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
@@ -241,6 +255,12 @@ def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, K
     out = softmax(q k^T * qk_scale) v * out_scale, the cached values taken without their global scales. `chunk` bounds
     the tokens that are held as 16-bit operands at a time; the scratch comes from torch's allocator. signs as in
     decode_ragged. The reference's counterpart is backend.py:438-543."""
+    rc = (_lib._host or _lib.host()).prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out,
+                                             chunk, k_f16, signs, k8, workspace)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "hkv_prefill")
+        return out
     if k8 and signs is not None:
         raise ValueError("the K8V4 slot keeps FP8 keys: no rotation")
     ready = query.dtype == torch.float16
