@@ -76,7 +76,7 @@ def load():
         L.hkv_prefill_scratch_bytes.argtypes = [C.POINTER(i32), i32, i32, i32, i32, i32, i64, i32]
         L.hkv_prefill.restype = i32
         L.hkv_prefill.argtypes = [vp, i32, vp, vp, vp, vp, C.POINTER(i64), i32, vp, i32, i32, C.POINTER(i32), i32, i32, i32,
-                                  i32, i32, f32, f32, i32, vp, i32, i64, vp, C.c_size_t, vp, i32, vp, vp]
+                                  i32, i32, f32, f32, vp, i32, i64, vp, C.c_size_t, vp, i32, vp, vp]
         L.hkv_selftest_wait_timeout.restype = i32
         L.hkv_selftest_wait_timeout.argtypes = [vp, i64, vp]
         L.hkv_selftest_codec.restype = i32

@@ -339,11 +339,12 @@ def _build_classes():
             """requests with more query tokens than the decode threshold, all in one call of the prefill kernels: their
             contexts (the new tokens were written by do_kv_cache_update) become 16-bit operands in chunks of
             HORIZON_KVFP4_CHUNK tokens (65,536, the reference's chunk: backend.py:16-25, :519-543), which bounds the
-            memory held. Causal window of the reference: query token t of ql sees keys j < L - ql + t + 1. Compute dtype
-            of the scores fp16 (HORIZON_KVFP4_PF16=1, the reference's default, backend.py:229: code * scale is exact in
-            fp16) or bf16; the value product takes fp16 operands (the dequantised values are exact in it and the
-            probabilities lie in [0, 2^8]); both accumulate in fp32. The global scales are folded into the softmax scale
-            and the output like the reference's sm / vs."""
+            memory held. Causal window of the reference: query token t of ql sees keys j < L - ql + t + 1. The score
+            product takes bf16 queries as they are (the reference's default converts them to fp16, backend.py:229; code *
+            scale is exact in both) and other types converted to fp16 (HORIZON_KVFP4_PF16=1) or bf16; the value product
+            takes fp16 operands (the dequantised values are exact in it and the probabilities lie in [0, 2^14]); both
+            accumulate in fp32. The global scales are folded into the softmax scale and the output like the reference's
+            sm / vs."""
             rows = [(row, q0, q1, L) for row, q0, q1, L in m.prefill_rows if q1 > q0 and L > 0]
             if not rows:
                 return
@@ -358,8 +359,8 @@ def _build_classes():
             o = out if direct else torch.empty(out.shape, dtype=torch.float32, device=out.device)
             bt = m.block_table if m.block_table.is_contiguous() else m.block_table.contiguous()
             K.prefill(q, v["flat"], v["strides"], v["PS"], bt, rows, self.scale * float(layer._k_scale_float),
-                      float(layer._v_scale_float), self.num_kv_heads, o, chunk=self.prefill_chunk, k_f16=self.pf16,
-                      signs=signs, k8=self.k8, workspace=self._state(q.device)["ws"])
+                      float(layer._v_scale_float), self.num_kv_heads, o, chunk=self.prefill_chunk, signs=signs, k8=self.k8,
+                      workspace=self._state(q.device)["ws"])
             if not direct:
                 for _, q0, q1, _ in rows:
                     out[q0:q1].copy_(o[q0:q1])

@@ -186,21 +186,21 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
-// prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out, chunk, k_f16, signs, k8, workspace)
+// prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out, chunk, signs, k8, workspace)
 PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
-    if (n != 15 || !abi.prefill) Py_RETURN_NONE;
-    const at::Tensor *q = tensor(a[0]), *bt = tensor(a[4]), *out = tensor(a[9]), *ws = a[14] == Py_None ? nullptr : tensor(a[14]);
-    if (!q || !bt || !out || (!ws && a[14] != Py_None) || !q->is_cuda() || !PyList_CheckExact(a[5])) Py_RETURN_NONE;
+    if (n != 14 || !abi.prefill) Py_RETURN_NONE;
+    const at::Tensor *q = tensor(a[0]), *bt = tensor(a[4]), *out = tensor(a[9]), *ws = a[13] == Py_None ? nullptr : tensor(a[13]);
+    if (!q || !bt || !out || (!ws && a[13] != Py_None) || !q->is_cuda() || !PyList_CheckExact(a[5])) Py_RETURN_NONE;
     const int dev = q->device().index();
     long long PS, KVH, chunk;
     double s1, s2;
-    bool k_f16, k8;
+    bool k8;
     const float* signs;
     Cache c;
     if (dev != c10::cuda::current_device() || !integer(a[3], &PS) || PS < 1 || PS != (int)PS || !number(a[6], &s1) ||
-        !number(a[7], &s2) || !integer(a[8], &KVH) || KVH < 1 || KVH != (int)KVH || !integer(a[10], &chunk) || !boolean(a[11], &k_f16) ||
-        !boolean(a[13], &k8))
+        !number(a[7], &s2) || !integer(a[8], &KVH) || KVH < 1 || KVH != (int)KVH || !integer(a[10], &chunk) ||
+        !boolean(a[12], &k8))
       Py_RETURN_NONE;
     const bool out_f32 = out->scalar_type() == at::kFloat;
     if (q->scalar_type() != at::kBFloat16 || (out->scalar_type() != at::kBFloat16 && !out_f32) || q->dim() != 3 || out->dim() != 3 ||
@@ -210,7 +210,7 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
       Py_RETURN_NONE;
     const int64_t B = bt->size(0), MP = bt->size(1), NT = q->size(0), HQ = q->size(1), D = q->size(2);
     if (HQ % KVH || B > INT32_MAX || MP > INT32_MAX || NT > INT32_MAX || HQ > INT32_MAX || D > INT32_MAX ||
-        !sign_vector(a[12], D, dev, &signs) || (k8 && signs) || !cache_of(a[1], a[2], dev, &c))
+        !sign_vector(a[11], D, dev, &signs) || (k8 && signs) || !cache_of(a[1], a[2], dev, &c))
       Py_RETURN_NONE;
     const Py_ssize_t n_rows = PyList_GET_SIZE(a[5]);
     if (n_rows > INT32_MAX) Py_RETURN_NONE;
@@ -235,8 +235,8 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = abi.prefill(qp, !signs && !k_f16, c.part[0], c.part[1], c.part[2], c.part[3], c.strides, (int)PS, btp, (int)B, (int)MP,
-                     rows.data(), (int)n_rows, (int)NT, (int)KVH, G, (int)D, (float)s1, (float)s2, k_f16, signs, k8, chunk, sp, nb, op,
+    rc = abi.prefill(qp, 0, c.part[0], c.part[1], c.part[2], c.part[3], c.strides, (int)PS, btp, (int)B, (int)MP,
+                     rows.data(), (int)n_rows, (int)NT, (int)KVH, G, (int)D, (float)s1, (float)s2, signs, k8, chunk, sp, nb, op,
                      out_f32, wp, st);
     Py_END_ALLOW_THREADS
     return PyLong_FromLong(rc);

@@ -10,11 +10,10 @@
 //
 // Replaces the reference's library attention over dequantised tokens (backend.py:438-543).
 //
-// Device times on a B200 (ncu, one launch alone; write launch included in the totals): a fresh prompt of 6144 tokens, 32
-// query heads over 8 kv heads, head_dim 128: tile 12 us, attend 308 us (1.0 PFLOP/s), merge 9 us; the layer step 366 us
-// against 16.5 ms with torch matmuls and eager softmax passes, whose fp32 score matrices went through memory. 2048 tokens
-// over 30000 cached, 16 heads over 2, head_dim 256: tile 28 us, attend 683 us (1.54 PFLOP/s), merge 10 us; the step 0.84
-// ms (the power cap lowers the clock) against 15.0 ms.
+// Layer steps on a B200 (write launch included): a fresh prompt of 6144 tokens, 32 query heads over 8 kv heads, head_dim 128:
+// 361 us (tile 12, attend about 295, merge 7) against 16.5 ms with torch matmuls and eager softmax passes, whose fp32 score
+// matrices went through memory. 2048 tokens over 30000 cached, 16 heads over 2, head_dim 256: 0.85 ms, at which the board
+// draws its 1000 W and the clock falls to 1.6 GHz (1.25 PFLOP/s; a plain bf16 GEMM sustains 1.37), against 15.0 ms.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -29,21 +28,20 @@ constexpr int kPfCtas = 160;           // CTAs per launch
 constexpr int kKeys = 128;             // keys per tile
 constexpr int kPieceCost = 3;          // cost of starting and ending a piece, in key tiles (of about 1 us)
 constexpr int kMinPiece = 2;           // no piece of a divided row tile is shorter, in key tiles
+constexpr float kMaxLag = 14.0f;        // log2 by which a score may exceed the running maximum: probabilities stay inside f16
 constexpr int kStageBytes = 32768;
 constexpr int kStages = 5;
-constexpr int kPfThreads = 320;        // 8 softmax warps, the MMA warp, the copy warp
-constexpr uint32_t kQBytes = 65536;    // query operands: 256 rows x 128 or 128 rows x 256 channels, 16 bits
+constexpr uint32_t kQBytes = 65536;    // query operands of 128 rows: two buffers at head_dim 128, one at 256
 
-// rows of the tensor-core tiles: a "piece row tile" has NT sub-tiles of 128 rows; row r of a sub-tile is query head
-// r % G of token r / G, so that a sub-tile covers 128 / G consecutive tokens and its causal edge is short
+// A row tile has 128 rows; row r is query head r % G of token r / G, so that it covers 128 / G consecutive tokens and its
+// causal edge is short.
 template <int D>
 struct PfShape {
-  static constexpr int NT = D == 128 ? 2 : 1;
-  static constexpr int ROWS = NT * 128;
-  static constexpr int COLS = D == 128 ? 128 : 64;      // score columns of a softmax thread
-  static constexpr int OCOL = 256;                      // tensor-memory column of the output accumulators
-  static constexpr int PCOL = D == 128 ? 64 : 0;        // probabilities, from the thread's first score column
-  static constexpr int PHALF = D == 128 ? 32 : 64;      // columns from the first 64 keys' probabilities to the others'
+  static constexpr int SETS = D == 128 ? 3 : 2;         // score tiles in flight, each with its softmax warpgroup
+  static constexpr int OCOL = SETS * 128;               // tensor-memory column of the output accumulator
+  static constexpr int NQ = D == 128 ? 2 : 1;           // query buffers
+  static constexpr int SOFT = 4 * SETS;                 // softmax warps
+  static constexpr int THREADS = 32 * (SOFT + 8);       // + the MMA warp, the copy warp, two idle ones; four end warps
 };
 
 struct PfReq {
@@ -62,15 +60,14 @@ struct PrefillParams {
   const void* q;
   void* out;
   const uint8_t* tiles;
-  float* part_o;                       // [CTA][2][ROWS][D]
-  float* part_ml;                      // [CTA][2][2][ROWS]: running maximum (log2 domain), sum
+  float* part_o;                       // [CTA][2][128][D]
+  float* part_ml;                      // [CTA][2][2][128]: running maximum (log2 domain), sum
   float* state_o;                      // chunked contexts: [token][head][D], then the same tables per row
   float* state_ml;
   int* status;
   float c, vs;                         // score scale x log2(e) (> 0), output scale
-  uint32_t q_flip;                     // 0x80008000 when the score scale is negative
-  int q_cvt, out_f32, k_bf16;
-  int KVH, G, tok;                     // tok: query tokens per sub-tile (128 / G)
+  int out_f32, k_bf16;
+  int KVH, G, tok;                     // tok: query tokens per row tile (128 / G)
   int n_req;
   int kt_lo, kt_hi;                    // key tiles of this launch's chunk
   int first_chunk;
@@ -82,25 +79,25 @@ static_assert(sizeof(PrefillParams) <= 4096, "kernel arguments");
 
 // one past the last key tile (of the chunk) that a row tile sees; at least one tile, so that rows without any visible
 // key still get their zero output
-__host__ __device__ inline int pf_hi(const PfReq& r, int rt, int piece_tok, int kt_hi) {
-  const int t_end = min(r.ql, (rt + 1) * piece_tok);
+__host__ __device__ inline int pf_hi(const PfReq& r, int rt, int tok, int kt_hi) {
+  const int t_end = min(r.ql, (rt + 1) * tok);
   const int vis = max(1, min(r.L, r.L - r.ql + t_end));
   return min((vis + kKeys - 1) / kKeys, kt_hi);
 }
-__host__ __device__ inline int pf_row_tiles(const PfReq& r, int piece_tok) { return (r.ql + piece_tok - 1) / piece_tok; }
+__host__ __device__ inline int pf_row_tiles(const PfReq& r, int tok) { return (r.ql + tok - 1) / tok; }
 
 struct Walk {
   int req, h, rt, kt;
   __host__ __device__ bool same_tile(const PfStart& e) const { return req == e.req && h == e.h && rt == e.rt; }
   // the next row tile that has keys in this chunk
-  __host__ __device__ void advance(const PfReq* r, int n_req, int KVH, int piece_tok, int kt_lo, int kt_hi) {
+  __host__ __device__ void advance(const PfReq* r, int n_req, int KVH, int tok, int kt_lo, int kt_hi) {
     kt = kt_lo;
     do {
-      if (++rt >= pf_row_tiles(r[req], piece_tok)) {
+      if (++rt >= pf_row_tiles(r[req], tok)) {
         rt = 0;
         if (++h >= KVH) { h = 0; ++req; }
       }
-    } while (req < n_req && pf_hi(r[req], rt, piece_tok, kt_hi) <= kt_lo);
+    } while (req < n_req && pf_hi(r[req], rt, tok, kt_hi) <= kt_lo);
   }
 };
 
@@ -115,6 +112,7 @@ struct TileParams {
   uint8_t* tiles;
   int MP, PS, KVH, n_req;
   int kt_lo, n_tiles;                  // first key tile of the chunk; key tiles of the launch
+  uint32_t k_flip;                     // 0x80008000 when the score scale is negative: the keys carry its sign
   int row[kPfReqs];                    // block-table rows
   int L[kPfReqs];
   int tile0[kPfReqs];
@@ -179,6 +177,8 @@ __global__ void __launch_bounds__(128) tile_kernel(const __grid_constant__ TileP
           }
         }
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] ^= p.k_flip;
       uint8_t* rowp = dst + (size_t)kb * 16384 + key * 128;
       *reinterpret_cast<uint4*>(rowp + (((blk4 * 2) ^ (key & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
       *reinterpret_cast<uint4*>(rowp + (((blk4 * 2 + 1) ^ (key & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
@@ -226,11 +226,11 @@ __global__ void __launch_bounds__(128) tile_kernel(const __grid_constant__ TileP
 
 // ------------------------------------------------------------------------------------------------- rotated queries
 // bf16 query rows -> bf16(FWHT(q * signs) * D^-0.5), butterflies in fp32 in the reference's stage order (rotate_q,
-// kv_fp4_ref.py:76-92, bit for bit) -> the compute type. One warp per row: a lane holds D / 32 adjacent channels, the
+// kv_fp4_ref.py:76-92, bit for bit). One warp per row: a lane holds D / 32 adjacent channels, the
 // first stages stay inside the lane, the others exchange between lanes.
 template <int D>
 __global__ void __launch_bounds__(256) rotate_kernel(const __nv_bfloat16* q, const float* signs, uint32_t* out, long long rows,
-                                                     float scale, int to_bf16) {
+                                                     float scale) {
   constexpr int V = D / 32;
   pdl_wait();
   pdl_launch_dependents();
@@ -259,8 +259,7 @@ __global__ void __launch_bounds__(256) rotate_kernel(const __nv_bfloat16* q, con
 #pragma unroll
   for (int i = 0; i < V; i += 2) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(x[i] * scale, x[i + 1] * scale);
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(&b);
-    out[(row * D + lane * V + i) / 2] = to_bf16 ? w : pack_f16x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    out[(row * D + lane * V + i) / 2] = *reinterpret_cast<const uint32_t*>(&b);
   }
 }
 
@@ -308,9 +307,19 @@ __device__ __forceinline__ void tm_ld32(uint32_t* x, uint32_t addr) {
       : HKV_R32(x)
       : "r"(addr));
 }
+__device__ __forceinline__ void tm_ld16(uint32_t* x, uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
+                 "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+               : "r"(addr));
+}
 __device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // keeps the uses of loaded registers behind the wait (an empty statement that passes them through)
 __device__ __forceinline__ void tm_ready(uint32_t* x) { asm volatile("" : HKV_RW32(x)); }
+__device__ __forceinline__ void tm_ready16(uint32_t* x) {
+  asm volatile("" : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(x[8]),
+                    "+r"(x[9]), "+r"(x[10]), "+r"(x[11]), "+r"(x[12]), "+r"(x[13]), "+r"(x[14]), "+r"(x[15]));
+}
 __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t* x) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::HKV_I16(x),
@@ -337,16 +346,26 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
   return r;
 }
 
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 struct PfShared {
   uint64_t full[kStages], empty[kStages];
-  uint64_t q_full[2], s_full[2], p_full[2], o_done[2];
-  uint64_t pair[4];                    // head_dim 256: the two warps that share 32 rows exchange maxima and sums
+  uint64_t q_full[2], q_free[2];       // query operands written / read for the last time in a piece
+  uint64_t s_full[3], p_full[3];       // [set] scores, probabilities
+  uint64_t o_done[3];                  // [set] value product of the set's tile has left the tensor pipe
+  uint64_t told[12];                   // [set][quad] running maxima of 32 rows
+  uint64_t ml_full, ml_free;           // a piece's maxima and sums written / read
+  uint64_t o_free;                     // a piece's output has left the accumulator
   uint64_t drain;
   uint32_t tmem;
   int abort;
 };
-constexpr int kPfSmem = (int)kQBytes + kStages * kStageBytes + 2048 + 512;
-static_assert(sizeof(PfShared) <= 512 && kPfSmem <= 232448, "shared memory");
+constexpr int kAux = (3 + 2) * 128 * 4;          // sums [set][128], running maxima [piece & 1][128]
+constexpr int kPfSmem = (int)kQBytes + kStages * kStageBytes + kAux + (int)sizeof(PfShared);
+static_assert(kPfSmem <= 232448, "shared memory");
 
 // bounded wait: gives up when it runs out or when another role of the CTA has given up
 __device__ __forceinline__ bool pf_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort) {
@@ -385,40 +404,106 @@ __device__ __forceinline__ void store_out(const PrefillParams& p, long long elem
 // kPieceCost per piece), so that a chunk of 2048 tokens over 30k keys and four short prompts both occupy every SM to
 // the end; a row tile whose keys were divided leaves unnormalised fp32 parts for merge_kernel.
 //
-// head_dim 128: two sub-tiles of 128 rows; while one has its scores exponentiated the tensor core works on the other.
-//   tensor memory: S0 S1 O0 O1, 128 columns each.
-// head_dim 256: one sub-tile (its output takes 256 columns), two score buffers; each score tile is shared by two
-//   softmax warpgroups, 64 columns each, which agree on the row maximum through shared memory.
-// Bound: tensor pipe and ex2 unit (16 per clock and SM: 1024 clocks per 128 x 128 scores, as long as the two products of
-// head_dim 128, half as long as those of head_dim 256, which therefore reaches 0.92 of the burst peak and the other 0.60).
-// The 16-bit probabilities overwrite their own scores in tensor memory. The running maximum moves only when a score
-// exceeds it by 2^8 (the probabilities then stay below 2^8, inside f16), so the output is rarely rescaled.
+// Roles: a copy warp streams key and value tiles through a ring; one thread issues all products; SETS warpgroups take the
+// score tiles in turn (a thread has a whole row of 128 scores); four end warps fetch the queries of the pieces to come and
+// write the outputs of the pieces that are done. Tensor memory: SETS score tiles of 128 columns, the output (head_dim
+// columns). Scores run SETS - 1 tiles ahead of the value products, across pieces too.
+//
+// Why so: a score tile is 1024 clocks of exponentials (ex2: 16 per clock and SM) and twice that again in latencies (loads
+// from tensor memory, barriers, contention) before its value product can start, while the tensor pipe needs 1024 clocks
+// (head_dim 128) or 2048 for both products. Two 128-row sub-tiles with one score buffer each left the tensor pipe idle 45 %
+// of the time (3590 clocks for both against 2048; here 1450 a tile) and 9000 clocks between pieces (here about 3000; short
+// prompts gain most, a step of four prompts with 48 decode requests went from 128 to 117 us); 64-key steps with two buffers
+// each paid twice for the score product, which reads its 128 query rows from shared memory whatever the number of keys.
+// The 16-bit probabilities go over the scores they came from. The running maximum moves only when a score exceeds it by
+// 2^14 (the probabilities then stay below 2^14, inside f16), so the output is hardly ever rescaled; a thread tells the next
+// tile's thread of its row the maximum as soon as it knows it.
+// A walk over the CTA's key tiles, piece by piece. A step to the next row tile of a request costs a few instructions: every
+// role takes it at every piece, two of them in a single thread.
+struct Tiles {
+  const PrefillParams& p;
+  PfStart last;
+  int req, h, rt, kt, hi;              // hi: end of the current piece
+  PfReq r;
+  int n_rt;                            // row tiles of the request
+  uint32_t piece;
+  bool first, end;                     // first tile of its piece; nothing left
+  __device__ __forceinline__ explicit Tiles(const PrefillParams& p_) : p(p_), last(p_.start[blockIdx.x + 1]), piece(0) {
+    const PfStart s = p_.start[blockIdx.x];
+    req = s.req;
+    h = s.h;
+    rt = s.rt;
+    kt = s.kt;
+    enter_request();
+    enter();
+  }
+  __device__ __forceinline__ void enter_request() {
+    if (req < p.n_req) {
+      r = p.req[req];
+      n_rt = pf_row_tiles(r, p.tok);
+    }
+  }
+  __device__ __forceinline__ bool cut() const { return rt == last.rt && h == last.h && req == last.req; }   // goes on in the next CTA
+  __device__ __forceinline__ int tile_hi() const { return pf_hi(r, rt, p.tok, p.kt_hi); }
+  __device__ __forceinline__ void enter() {
+    first = true;
+    const bool c = cut();
+    end = c && kt >= last.kt;
+    hi = c ? last.kt : tile_hi();
+  }
+  __device__ __forceinline__ void next_piece() {
+    if (cut()) {
+      end = true;
+      return;
+    }
+    kt = p.kt_lo;
+    do {
+      if (++rt >= n_rt) {
+        rt = 0;
+        if (++h >= p.KVH) {
+          h = 0;
+          ++req;
+          enter_request();
+        }
+      }
+    } while (req < p.n_req && tile_hi() <= p.kt_lo);      // (no keys in this chunk)
+    ++piece;
+    enter();
+  }
+  __device__ __forceinline__ void next() {
+    first = false;
+    if (++kt == hi) next_piece();
+  }
+};
+
 template <int D>
-__global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_constant__ PrefillParams p) {
+__global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __grid_constant__ PrefillParams p) {
   using S = PfShape<D>;
-  constexpr int COLS = S::COLS;
+  constexpr int SETS = S::SETS, SOFT = S::SOFT, NQ = S::NQ;
+  constexpr uint32_t IMAGE = kKeys * D * 2;
+  constexpr int PER = IMAGE / kStageBytes;                // ring stages per operand tile: 1 or 2
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* ring = smem + kQBytes;
-  float* xch = reinterpret_cast<float*>(smem + kQBytes + kStages * kStageBytes);      // [2 turns][2 halves][128 rows]
-  PfShared& sh = *reinterpret_cast<PfShared*>(smem + kQBytes + kStages * kStageBytes + 2048);
+  uint8_t* aux = smem + kQBytes + kStages * kStageBytes;
+  volatile float* xl = reinterpret_cast<float*>(aux);               // [set][128]: sums of a piece
+  volatile float* xm = reinterpret_cast<float*>(aux) + 3 * 128;     // [piece & 1][128]: running maxima (log2 domain)
+  PfShared& sh = *reinterpret_cast<PfShared*>(aux + kAux);
   volatile int* abort = &sh.abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int piece_tok = S::NT * p.tok;
 
   if (tid == 0) {
     sh.abort = (smem_u32(smem) & 1023) ? 1 : 0;        // the swizzled operands need 1024-byte alignment
     for (int i = 0; i < kStages; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.q_full[i], S::NT == 2 ? 128 : 256);
-      mbar_init(&sh.s_full[i], 1);
-      mbar_init(&sh.p_full[i], S::NT == 2 ? 128 : 256);
-      mbar_init(&sh.o_done[i], 1);
-    }
-    for (int i = 0; i < 4; ++i) mbar_init(&sh.pair[i], 64);
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.q_full[i], 128); mbar_init(&sh.q_free[i], 1); }
+    for (int i = 0; i < 3; ++i) { mbar_init(&sh.s_full[i], 1); mbar_init(&sh.p_full[i], 128); mbar_init(&sh.o_done[i], 1); }
+    for (int i = 0; i < 12; ++i) mbar_init(&sh.told[i], 32);
+    mbar_init(&sh.ml_full, SETS * 128);
+    mbar_init(&sh.ml_free, 128);
+    mbar_init(&sh.o_free, 128);
     mbar_init(&sh.drain, 1);
     fence_barrier_init();
   }
-  if (warp == 8) {
+  if (warp == SOFT) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&sh.tmem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
@@ -429,362 +514,174 @@ __global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_cons
   pdl_wait();
   pdl_launch_dependents();
 
-  const PfStart first = p.start[blockIdx.x], last = p.start[blockIdx.x + 1];
-  Walk w{first.req, first.h, first.rt, first.kt};
   const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]), q_full0 = smem_u32(&sh.q_full[0]),
-                 s_full0 = smem_u32(&sh.s_full[0]), p_full0 = smem_u32(&sh.p_full[0]), o_done0 = smem_u32(&sh.o_done[0]);
+                 q_free0 = smem_u32(&sh.q_free[0]), s_full0 = smem_u32(&sh.s_full[0]), p_full0 = smem_u32(&sh.p_full[0]),
+                 o_done0 = smem_u32(&sh.o_done[0]), told0 = smem_u32(&sh.told[0]), ml_full = smem_u32(&sh.ml_full),
+                 ml_free = smem_u32(&sh.ml_free), o_free = smem_u32(&sh.o_free);
+  auto all_wait = [&](uint32_t bar, uint32_t phase) { return (bool)__all_sync(0xffffffffu, pf_wait(bar, phase & 1, abort)); };
 
-  if (warp == 9) {
+  if (warp == SOFT + 1) {
     // ------------------------------------------------------------------------------------------------ copy warp
     if (elect_one()) {
-      constexpr uint32_t IMAGE = kKeys * D * 2;
-      constexpr int PER = IMAGE / kStageBytes;            // stages per operand tile: 1 or 2
-      uint32_t fill = 0;
+      Tiles k(p), v(p);
+      uint32_t fill = 0, st = 0, turn = 0;
       bool ok = *abort == 0;
-      while (ok && (!w.same_tile(last) || w.kt < last.kt)) {
-        const PfReq r = p.req[w.req];
-        const int hi = w.same_tile(last) ? last.kt : pf_hi(r, w.rt, piece_tok, p.kt_hi);
+      auto fetch = [&](Tiles& x, int side) {
+        const PfReq& r = x.r;
         const int n_t = min(p.kt_hi, (r.L + kKeys - 1) / kKeys) - p.kt_lo;
-        const uint8_t* src = p.tiles + ((size_t)r.tile0 * p.KVH + (size_t)w.h * n_t - p.kt_lo) * 2 * IMAGE;
-        auto fetch = [&](const uint8_t* from) {
-          for (int i = 0; ok && i < PER; ++i) {
-            const uint32_t st = fill % kStages, turn = fill / kStages;
-            if (turn > 0) ok = pf_wait(empty0 + 8 * st, (turn - 1) & 1, abort);
-            if (!ok) return;
-            mbar_expect_tx_u32(full0 + 8 * st, kStageBytes);
-            bulk_g2s_u32(smem_u32(ring) + st * kStageBytes, from + i * kStageBytes, kStageBytes, full0 + 8 * st);
-            ++fill;
-          }
-        };
-        fetch(src + (size_t)w.kt * 2 * IMAGE);
-        for (int kt = w.kt; ok && kt < hi; ++kt) {
-          if (kt + 1 < hi) fetch(src + (size_t)(kt + 1) * 2 * IMAGE);
-          fetch(src + (size_t)kt * 2 * IMAGE + IMAGE);
+        const uint8_t* from = p.tiles + ((size_t)r.tile0 * p.KVH + (size_t)x.h * n_t + (x.kt - p.kt_lo)) * 2 * IMAGE + side * IMAGE;
+        for (int i = 0; ok && i < PER; ++i) {
+          if (turn > 0) ok = pf_wait(empty0 + 8 * st, (turn - 1) & 1, abort);
+          if (!ok) return;
+          mbar_expect_tx_u32(full0 + 8 * st, kStageBytes);
+          bulk_g2s_u32(smem_u32(ring) + st * kStageBytes, from + i * kStageBytes, kStageBytes, full0 + 8 * st);
+          ++fill;
+          if (++st == kStages) { st = 0; ++turn; }
         }
-        if (w.same_tile(last)) break;
-        w.advance(p.req, p.n_req, p.KVH, piece_tok, p.kt_lo, p.kt_hi);
+        x.next();
+      };
+      for (int i = 0; ok && i < SETS - 1 && !k.end; ++i) fetch(k, 0);
+      while (ok && !v.end) {
+        if (!k.end) fetch(k, 0);
+        if (ok) fetch(v, 1);
       }
       if (!ok) {                       // nothing of this CTA's may still be on its way when it ends
         for (uint32_t f = fill > kStages ? fill - kStages : 0; f < fill; ++f)
           mbar_wait_bounded_u32(full0 + 8 * (f % kStages), (f / kStages) & 1);
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == SOFT) {
     // ------------------------------------------------------------------------------------------------- MMA warp
     if (elect_one()) {
       const uint32_t base = (1u << 4) | ((128u / 16) << 24);
-      const uint32_t id_qk = base | ((128u / 8) << 17) | (p.k_bf16 ? (1u << 7) | (1u << 10) : 0u);
+      const uint32_t id_qk = base | ((uint32_t)(kKeys / 8) << 17) | (p.k_bf16 ? (1u << 7) | (1u << 10) : 0u);
       const uint32_t id_pv = base | ((uint32_t)(D / 8) << 17);
       const uint32_t q_smem = smem_u32(smem), ring_a = smem_u32(ring);
-      uint32_t use = 0, g = 0, piece = 0;                 // stages consumed, key tiles done, pieces done
+      Tiles k(p), v(p);
+      uint32_t use = 0;                                   // ring stages handed out, in the copy warp's order
+      uint32_t sk = 0, sv = 0, tv = 0;                    // score tile (of SETS) of the next score and value product; turn of the latter
       bool ok = *abort == 0;
       auto stage_wait = [&](uint32_t n) { return pf_wait(full0 + 8 * (n % kStages), (n / kStages) & 1, abort); };
       auto stage_addr = [&](uint32_t n) { return ring_a + (n % kStages) * kStageBytes; };
-      // scores of a sub-tile: K tile in stages n (and n + 1)
-      auto qk = [&](int sub, uint32_t n, uint32_t col) {
+      auto stages_done = [&](uint32_t n) {
+        for (int i = 0; i < PER; ++i) umma_commit(empty0 + 8 * ((n + i) % kStages));
+      };
+      auto scores = [&](uint32_t n) {                     // of the next key tile, which lies in stage n (and n + 1)
+        const uint32_t qb = k.piece % NQ;
+        if (k.first) ok = pf_wait(q_full0 + 8 * qb, (k.piece / NQ) & 1, abort);
+        ok = ok && stage_wait(n) && (PER == 1 || stage_wait(n + 1));
+        if (!ok) return;
+        tc_fence_after();
 #pragma unroll
         for (int kb = 0; kb < D / 64; ++kb) {
-          const uint64_t a = umma_desc(q_smem + sub * 32768 + kb * 16384);
+          const uint64_t a = umma_desc(q_smem + qb * 32768 + kb * 16384);
           const uint64_t b = umma_desc(stage_addr(n + kb / 2) + (kb & 1) * 16384);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_ss(tmem + col, a + 2 * k, b + 2 * k, id_qk, kb + k > 0);
+          for (int i = 0; i < 4; ++i) umma_ss(tmem + sk * 128, a + 2 * i, b + 2 * i, id_qk, kb + i > 0);
         }
+        umma_commit(s_full0 + 8 * sk);
+        stages_done(n);
+        if (k.kt + 1 == k.hi) umma_commit(q_free0 + 8 * qb);
+        if (++sk == SETS) sk = 0;
+        k.next();
       };
-      auto pv = [&](uint32_t pcol, uint32_t n, uint32_t ocol, bool acc) {
+      auto values = [&](uint32_t n) {
+        // (the accumulator holds the piece before until the end warps have read it)
+        ok = stage_wait(n) && (PER == 1 || stage_wait(n + 1)) &&
+             (!v.first || v.piece == 0 || pf_wait(o_free, (v.piece - 1) & 1, abort)) && pf_wait(p_full0 + 8 * sv, tv & 1, abort);
+        if (!ok) return;
+        tc_fence_after();
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb) {
-          const uint64_t b = umma_desc(D == 128 ? stage_addr(n) + kb * 16384 : stage_addr(n + kb));
+          const uint64_t b = umma_desc(PER == 1 ? stage_addr(n) + kb * 16384 : stage_addr(n + kb));
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ts(tmem + ocol, tmem + pcol + S::PCOL + kb * S::PHALF + k * 8, b + 2 * k, id_pv, acc || kb + k > 0);
+          for (int i = 0; i < 4; ++i)
+            umma_ts(tmem + S::OCOL, tmem + sv * 128 + 64 + kb * 32 + i * 8, b + 2 * i, id_pv, !v.first || kb + i > 0);
         }
+        umma_commit(o_done0 + 8 * sv);
+        stages_done(n);
+        if (++sv == SETS) { sv = 0; ++tv; }
+        v.next();
       };
-      while (ok && (!w.same_tile(last) || w.kt < last.kt)) {
-        const int hi = w.same_tile(last) ? last.kt : pf_hi(p.req[w.req], w.rt, piece_tok, p.kt_hi);
-        const int n = hi - w.kt;
-        if constexpr (D == 128) {
-          ok = stage_wait(use);
-          for (int t = 0; ok && t < 2; ++t) {
-            ok = pf_wait(q_full0 + 8 * t, piece & 1, abort);
-            if (!ok) break;
-            tc_fence_after();
-            qk(t, use, t * 128);
-            umma_commit(s_full0 + 8 * t);
-          }
-          if (ok) umma_commit(empty0 + 8 * (use % kStages));
-          ++use;
-          for (int j = 0; ok && j < n; ++j, ++g) {
-            const bool more = j + 1 < n;
-            const uint32_t kst = use, vst = use + (more ? 1 : 0);
-            use = vst + 1;
-            for (int t = 0; ok && t < 2; ++t) {
-              if (t == 0) ok = stage_wait(vst);
-              ok = ok && pf_wait(p_full0 + 8 * t, g & 1, abort);
-              if (!ok) break;
-              tc_fence_after();
-              pv(t * 128, vst, S::OCOL + t * 128, j > 0);
-              umma_commit(o_done0 + 8 * t);
-              if (more) {
-                if (t == 0) ok = stage_wait(kst);
-                if (!ok) break;
-                qk(t, kst, t * 128);
-                umma_commit(s_full0 + 8 * t);
-              }
-            }
-            if (ok) {
-              if (more) umma_commit(empty0 + 8 * (kst % kStages));
-              umma_commit(empty0 + 8 * (vst % kStages));
-            }
-          }
-        } else {
-          ok = pf_wait(q_full0, piece & 1, abort) && stage_wait(use) && stage_wait(use + 1);
-          if (ok) {
-            tc_fence_after();
-            qk(0, use, (g & 1) * 128);
-            umma_commit(s_full0 + 8 * (g & 1));
-            umma_commit(empty0 + 8 * (use % kStages));
-            umma_commit(empty0 + 8 * ((use + 1) % kStages));
-          }
-          use += 2;
-          for (int j = 0; ok && j < n; ++j, ++g) {
-            if (j + 1 < n) {
-              ok = stage_wait(use) && stage_wait(use + 1);
-              if (!ok) break;
-              qk(0, use, ((g + 1) & 1) * 128);
-              umma_commit(s_full0 + 8 * ((g + 1) & 1));
-              umma_commit(empty0 + 8 * (use % kStages));
-              umma_commit(empty0 + 8 * ((use + 1) % kStages));
-              use += 2;
-            }
-            ok = stage_wait(use) && stage_wait(use + 1) && pf_wait(p_full0 + 8 * (g & 1), (g >> 1) & 1, abort);
-            if (!ok) break;
-            tc_fence_after();
-            pv((g & 1) * 128, use, S::OCOL, j > 0);
-            umma_commit(o_done0 + 8 * (g & 1));
-            umma_commit(empty0 + 8 * (use % kStages));
-            umma_commit(empty0 + 8 * ((use + 1) % kStages));
-            use += 2;
-          }
+      for (int i = 0; ok && i < SETS - 1 && !k.end; ++i) { scores(use); use += PER; }
+      while (ok && !v.end) {
+        if (k.end) {
+          values(use);
+          use += PER;
+          continue;
         }
-        ++piece;
-        if (w.same_tile(last)) break;
-        w.advance(p.req, p.n_req, p.KVH, piece_tok, p.kt_lo, p.kt_hi);
+        // (a single query buffer is only refilled once the scores of the piece are done: the value product does not wait)
+        const bool later = NQ == 1 && k.first;
+        if (later) values(use + PER);
+        if (ok) scores(use);
+        if (ok && !later) values(use + PER);
+        use += 2 * PER;
       }
       if (!ok) {                       // no product of this CTA's may still be running when its tensor memory is given back
         umma_commit(smem_u32(&sh.drain));
         mbar_wait_bounded_u32(smem_u32(&sh.drain), 0);
       }
     }
-  } else {
-    // -------------------------------------------------------------------------------------------- softmax warps
-    const int wg = warp >> 2, quad = warp & 3;
-    const int row = quad * 32 + lane;                     // of the sub-tile, = tensor-memory lane
-    const int sub = D == 128 ? wg : 0;
-    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-    const uint32_t o_addr = lane_base + S::OCOL + wg * 128;
-    const uint32_t pair_bar = smem_u32(&sh.pair[quad]);
-    const uint32_t q_bar = q_full0 + 8 * sub;
-    uint32_t turn = 0, g = 0;                             // exchanges done, key tiles done
+  } else if (warp >= SOFT + 4) {
+    // ------------------------------------------------------------------------------------------------ end warps
+    const int row = tid - (SOFT + 4) * 32, quad = warp & 3;              // row of the tile, = tensor-memory lane
+    const uint32_t inv_g = 65536u / p.G + 1;              // floor(row / G) = row * inv_g >> 16 for rows below 128
+    const int HQ = p.KVH * p.G;
+    Tiles x(p), y(p);                                  // the piece to write out; the piece to fetch queries of
+    uint32_t g = 0;
     bool ok = *abort == 0;
-
-    auto load_q = [&](const Walk& x) {
-      // this warpgroup's (head_dim 256: both warpgroups') rows, 16 bytes per lane and load, whole rows per half warp or warp
-      constexpr int LPR = D / 8;                          // lanes per row
-      constexpr int NTH = D == 128 ? 128 : 256;
-      const PfReq r = p.req[x.req];
-      const int t = D == 128 ? (tid & 127) : tid;
-      const int ch = t % LPR;
-      uint8_t* qs = smem + sub * 32768 + (ch >> 3) * 16384;
-      const int tok0 = x.rt * piece_tok + sub * p.tok;
-      const int HQ = p.KVH * p.G;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rr = t / LPR + (half * 8 + i) * (NTH / LPR);
-          const int tk = rr / p.G, token = tok0 + tk;
-          v[i] = make_uint4(0, 0, 0, 0);
-          if (tk < p.tok && token < r.ql) {
-            const long long e = ((long long)(r.q0 + token) * HQ + x.h * p.G + (rr - tk * p.G)) * D + ch * 8;
-            v[i] = *reinterpret_cast<const uint4*>((const uint16_t*)p.q + e);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rr = t / LPR + (half * 8 + i) * (NTH / LPR);
-          uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            u[k] ^= p.q_flip;
-            if (p.q_cvt) u[k] = pack_f16x2(__uint_as_float(u[k] << 16), __uint_as_float(u[k] & 0xffff0000u));
-          }
-          *reinterpret_cast<uint4*>(qs + rr * 128 + (((ch & 7) ^ (rr & 7)) << 4)) = make_uint4(u[0], u[1], u[2], u[3]);
-        }
+    // queries of piece y: 16 bytes per lane and copy, whole rows per half warp or warp; rows that do not exist are zero
+    auto load_q = [&]() {
+      constexpr int LPR = D / 8, RSTEP = 128 / LPR;
+      const PfReq r = y.r;
+      const int ch = row % LPR, tok0 = y.rt * p.tok;
+      const uint32_t qs = smem_u32(smem) + (y.piece % NQ) * 32768 + (ch >> 3) * 16384;
+      const uint16_t* q = (const uint16_t*)p.q + ((long long)(r.q0 + tok0) * HQ + y.h * p.G) * D + ch * 8;
+      if (y.piece >= NQ && !pf_wait(q_free0 + 8 * (y.piece % NQ), (y.piece / NQ - 1) & 1, abort)) return false;
+#pragma unroll 4
+      for (int rr = row / LPR; rr < 128; rr += RSTEP) {
+        const int tk = (int)((uint32_t)rr * inv_g >> 16);
+        const uint32_t dst = qs + rr * 128 + (((ch & 7) ^ (rr & 7)) << 4);
+        if (tk < p.tok && tok0 + tk < r.ql) cp_async<16>(dst, q + ((long long)tk * HQ + (rr - tk * p.G)) * D);
+        else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       fence_proxy_async();
-      mbar_arrive_u32(q_bar);
+      mbar_arrive_u32(q_full0 + 8 * (y.piece % NQ));
+      return true;
     };
-    // head_dim 256: this thread's value and that of the thread that holds the row's other columns
-    auto exchange = [&](float mine, float& other) {
-      float* buf = xch + (turn & 1) * 256;
-      buf[wg * 128 + row] = mine;
-      mbar_arrive_u32(pair_bar);
-      const bool good = __all_sync(0xffffffffu, pf_wait(pair_bar, turn & 1, abort));
-      other = *(volatile float*)&buf[(wg ^ 1) * 128 + row];
-      ++turn;
-      return good;
-    };
-
-    // the value product of key tile n has completed (head_dim 256: the scores of tile n + 1 precede it, so two barriers take
-    // turns, lest a wait meet a phase two behind)
-    auto o_wait = [&](uint32_t n) {
-      return __all_sync(0xffffffffu, D == 128 ? pf_wait(o_done0 + 8 * wg, n & 1, abort)
-                                              : pf_wait(o_done0 + 8 * (n & 1), (n >> 1) & 1, abort));
-    };
-
-    bool first_piece = true;
-    if (ok && (!w.same_tile(last) || w.kt < last.kt)) load_q(w);
-    while (ok && (!w.same_tile(last) || w.kt < last.kt)) {
-      const PfReq r = p.req[w.req];
-      const bool cut = w.same_tile(last);                 // the row tile goes on in the next CTA
-      const int tile_hi = pf_hi(r, w.rt, piece_tok, p.kt_hi);
-      const int hi = cut ? last.kt : tile_hi;
-      const int tk = row / p.G, gq = row - tk * p.G;
-      const int token = w.rt * piece_tok + sub * p.tok + tk;
+    for (int i = 0; ok && i < NQ && !y.end; ++i) {
+      ok = __all_sync(0xffffffffu, load_q());
+      y.next_piece();
+    }
+    while (ok && !x.end) {
+      if (!y.end) {
+        ok = __all_sync(0xffffffffu, load_q());
+        if (!ok) break;
+        y.next_piece();
+      }
+      const PfReq r = x.r;
+      const int tile_hi = x.tile_hi();
+      g += x.hi - x.kt;
+      const bool divided = x.cut() || x.kt > p.kt_lo;
+      const int tk = (int)((uint32_t)row * inv_g >> 16), token = x.rt * p.tok + tk;
       const bool live = tk < p.tok && token < r.ql;
-      const int lim = live ? max(0, min(r.L, r.L - r.ql + token + 1)) : 0;      // keys this row sees
-      // tiles below this one are seen whole by every live row of the sub-tile (rows that do not exist may take any value)
-      const int whole = max(0, min(r.L, r.L - r.ql + w.rt * piece_tok + sub * p.tok + 1)) / kKeys;
-      float m = -INFINITY;
-      unsigned long long l2 = 0;                          // two partial sums
-      for (int kt = w.kt; kt < hi; ++kt, ++g) {
-        const uint32_t sb = D == 128 ? (uint32_t)wg : (g & 1);
-        const uint32_t ph = D == 128 ? (g & 1) : ((g >> 1) & 1);
-        const uint32_t s_addr = lane_base + sb * 128 + (D == 128 ? 0 : wg * 64);
-        ok = __all_sync(0xffffffffu, pf_wait(s_full0 + 8 * sb, ph, abort));
-        if (!ok) break;
-        tc_fence_after();
-        const bool edge = kt >= whole;
-        const int rel = lim - kt * kKeys - (D == 128 ? 0 : wg * 64);
-        auto mask = [&](uint32_t* x, int col, int n) {    // scores of keys past the row's last one
-#pragma unroll
-          for (int i = 0; i < n; ++i)
-            if (col + i >= rel) x[i] = 0xff800000u;
-        };
-        uint32_t s[COLS];
-#pragma unroll
-        for (int i = 0; i < COLS; i += 32) tm_ld32(s + i, s_addr + i);
-        tm_wait_ld();
-#pragma unroll
-        for (int i = 0; i < COLS; i += 32) tm_ready(s + i);
-        if (edge) mask(s, 0, COLS);
-        float mx[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) mx[i] = __uint_as_float(s[i]);
-#pragma unroll
-        for (int i = 4; i < COLS; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(s[i]));
-        float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.c;
-        if constexpr (D == 256) {
-          float other;
-          ok = exchange(top, other);
-          if (!ok) break;
-          top = fmaxf(top, other);
-        }
-        const bool move = top > m + 8.0f;
-        if (__any_sync(0xffffffffu, move)) {
-          const float m_new = move ? (top == INFINITY ? 0.0f : top) : m;
-          const float al = move ? fast_exp2(m - m_new) : 1.0f;
-          m = m_new;
-          l2 = fma2(l2, pack2(al, al), 0ull);
-          if (kt > w.kt) {
-            // the last value product must have left the accumulator; the next waits for this warp's probabilities
-            ok = o_wait(g - 1);
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int i = 0; i < 128; i += 32) {
-              uint32_t o[32];
-              tm_ld32(o, o_addr + i);
-              tm_wait_ld();
-              tm_ready(o);
-#pragma unroll
-              for (int k = 0; k < 32; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * al);
-              tm_st16(o_addr + i, o);
-              tm_st16(o_addr + i + 16, o + 16);
-            }
-          }
-        }
-        const float mu = m == -INFINITY ? 0.0f : -m;
-        const unsigned long long c2 = pack2(p.c, p.c), m2 = pack2(mu, mu);
-        auto probs = [&](const uint32_t* x, uint32_t addr) {        // 32 scores -> 32 probabilities in 16 columns
-          uint32_t ph16[16];
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            float a, b;
-            unpack2(fma2(pack2(__uint_as_float(x[2 * k]), __uint_as_float(x[2 * k + 1])), c2, m2), a, b);
-            a = fast_exp2(a);
-            b = fast_exp2(b);
-            l2 = add2(l2, pack2(a, b));
-            ph16[k] = pack_f16x2(a, b);
-          }
-          tm_st16(addr, ph16);
-        };
-        if constexpr (D == 128) {
-          // the second half of the scores stays in registers and its probabilities go over the columns it came from; the
-          // first half is read once more (128 scores, their maximum and the packed results do not fit 168 registers)
-          uint32_t r[64];
-          tm_ld32(r, s_addr);
-          tm_ld32(r + 32, s_addr + 32);
-          probs(s + 64, s_addr + S::PCOL + 32);
-          probs(s + 96, s_addr + S::PCOL + 48);
-          tm_wait_ld();
-          tm_ready(r);
-          tm_ready(r + 32);
-          if (edge) mask(r, 0, 64);
-          probs(r, s_addr + S::PCOL);
-          probs(r + 32, s_addr + S::PCOL + 16);
-        } else {
-          probs(s, s_addr + S::PCOL);
-          probs(s + 32, s_addr + S::PCOL + 16);
-        }
-        tc_wait_st();
-        tc_fence_before();
-        mbar_arrive_u32(p_full0 + 8 * sb);
-      }
+      const int head = x.h * p.G + (row - tk * p.G);
+      ok = all_wait(ml_full, x.piece);
       if (!ok) break;
-      // the next piece's queries go in while the last value product runs (its scores have left the query operands)
-      const Walk done = w;
-      if (!cut) w.advance(p.req, p.n_req, p.KVH, piece_tok, p.kt_lo, p.kt_hi);
-      if (!cut && (!w.same_tile(last) || w.kt < last.kt)) load_q(w);
-      float l, l_hi;
-      unpack2(l2, l, l_hi);
-      l += l_hi;
-      if constexpr (D == 256) {
-        float other;
-        ok = exchange(l, other);
-        if (!ok) break;
-        l += other;
-      }
-      ok = o_wait(g - 1);
-      if (!ok) break;
-      tc_fence_after();
-      const bool divided = cut || done.kt > p.kt_lo;
-      const int HQ = p.KVH * p.G;
-      const int col0 = D == 128 ? 0 : wg * 128;
-      float wo = 0.0f, wn = 1.0f, inv = 0.0f;
-      long long st_row = 0;
+      float l = xl[row], m = xm[(x.piece & 1) * 128 + row];
+      for (int i = 1; i < SETS; ++i) l += xl[i * 128 + row];
+      mbar_arrive_u32(ml_free);
+      float wo = 0.0f, wn = 1.0f;
+      const long long st_row = (long long)token * HQ + head;
       bool finish = true;
       float* part = nullptr;
       if (divided) {
-        const long long slot = (long long)blockIdx.x * 2 + (first_piece ? 0 : 1);
-        part = p.part_o + (slot * S::ROWS + sub * 128 + row) * D + col0;
-        if (D == 128 || wg == 0) {
-          p.part_ml[(slot * 2) * S::ROWS + sub * 128 + row] = m;
-          p.part_ml[(slot * 2 + 1) * S::ROWS + sub * 128 + row] = l;
-        }
+        const long long slot = (long long)blockIdx.x * 2 + (x.piece == 0 ? 0 : 1);
+        part = p.part_o + (slot * 128 + row) * D;
+        p.part_ml[slot * 256 + row] = m;
+        p.part_ml[slot * 256 + 128 + row] = l;
       } else if (p.state_o != nullptr && live) {
-        st_row = (long long)token * HQ + done.h * p.G + gq;
         float mo = -INFINITY, lo = 0.0f;
         if (!p.first_chunk) {
           mo = p.state_ml[2 * st_row];
@@ -795,17 +692,59 @@ __global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_cons
         wn = fast_exp2(m - ms);
         l = l * wn + lo * wo;
         m = mm;
-        finish = tile_hi == (max(1, min(r.L, r.L - r.ql + min(r.ql, (done.rt + 1) * piece_tok))) + kKeys - 1) / kKeys;
+        finish = tile_hi == (max(1, min(r.L, r.L - r.ql + min(r.ql, (x.rt + 1) * p.tok))) + kKeys - 1) / kKeys;
+        if (!finish) {
+          p.state_ml[2 * st_row] = m;
+          p.state_ml[2 * st_row + 1] = l;
+        }
       }
-      inv = p.vs / fmaxf(l, 1e-30f);
+      float inv = p.vs / fmaxf(l, 1e-30f);
       if (l != l) inv = l;
-      const long long out_row = ((long long)(r.q0 + token) * HQ + done.h * p.G + gq) * D + col0;
+      const long long out_row = ((long long)(r.q0 + token) * HQ + head) * D;
+      ok = all_wait(o_done0 + 8 * ((g - 1) % SETS), (g - 1) / SETS);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t o_addr = tmem + ((uint32_t)(quad * 32) << 16) + S::OCOL;
+      if (!divided && p.state_o == nullptr && !p.out_f32) {
+        // the usual output: 16 bits, 64 columns at a time; the accumulator is free before the last ones are stored
+#pragma unroll 1
+        for (int i = 0; i < D; i += 64) {
+          uint32_t u[32];
 #pragma unroll
-      for (int i = 0; i < 128; i += 32) {
+          for (int k = 0; k < 2; ++k) {
+            uint32_t o[32];
+            tm_ld32(o, o_addr + i + 32 * k);
+            tm_wait_ld();
+            tm_ready(o);
+#pragma unroll
+            for (int n = 0; n < 16; ++n) {
+              const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(o[2 * n]) * inv, __uint_as_float(o[2 * n + 1]) * inv);
+              u[16 * k + n] = *reinterpret_cast<const uint32_t*>(&b);
+            }
+          }
+          if (i + 64 == D) {
+            tc_fence_before();
+            mbar_arrive_u32(o_free);
+          }
+          if (live) {
+            uint4* dst = reinterpret_cast<uint4*>((__nv_bfloat16*)p.out + out_row + i);
+#pragma unroll
+            for (int n = 0; n < 8; ++n) dst[n] = make_uint4(u[4 * n], u[4 * n + 1], u[4 * n + 2], u[4 * n + 3]);
+          }
+        }
+        x.next_piece();
+        continue;
+      }
+#pragma unroll 1
+      for (int i = 0; i < D; i += 32) {
         uint32_t o[32];
         tm_ld32(o, o_addr + i);
         tm_wait_ld();
         tm_ready(o);
+        if (i + 32 == D) {
+          tc_fence_before();
+          mbar_arrive_u32(o_free);
+        }
         if (divided) {
 #pragma unroll
           for (int k = 0; k < 32; k += 4) *reinterpret_cast<uint4*>(part + i + k) = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
@@ -814,7 +753,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_cons
 #pragma unroll
           for (int k = 0; k < 32; ++k) f[k] = __uint_as_float(o[k]);
           if (p.state_o != nullptr) {
-            float* so = p.state_o + st_row * D + col0 + i;
+            float* so = p.state_o + st_row * D + i;
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
               f[k] *= wn;
@@ -833,26 +772,142 @@ __global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_cons
           }
         }
       }
-      if (D == 256 && !divided && p.state_o != nullptr) {
-        // both threads of a row have read its old maximum and sum before one of them writes the new ones
-        float other;
-        ok = exchange(0.0f, other);
+      x.next_piece();
+    }
+  } else if (warp < SOFT) {
+    // -------------------------------------------------------------------------------------------- softmax warps
+    const int set = warp >> 2, quad = warp & 3;
+    const int row = quad * 32 + lane;                     // of the tile, = tensor-memory lane
+    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16), s_addr = lane_base + set * 128;
+    const uint32_t s_bar = s_full0 + 8 * set, my_word = told0 + 8 * (set * 4 + quad);
+    const int before = set == 0 ? SETS - 1 : set - 1;     // the set of the tile before
+    const uint32_t word_before = told0 + 8 * (before * 4 + quad);
+    Tiles x(p);
+    uint32_t g = set, turn = 0;                           // the set's next tile in the CTA's stream; its tiles done
+    uint32_t g0 = 0;                                      // first tile of the piece
+    const int tk = row / p.G;
+    bool ok = *abort == 0;
+    while (ok && !x.end) {
+      const PfReq& r = x.r;
+      const int token = x.rt * p.tok + tk;
+      const int lim = tk < p.tok && token < r.ql ? max(0, min(r.L, r.L - r.ql + token + 1)) : 0;      // keys this row sees
+      // keys below this one are seen by every live row of the tile (rows that do not exist may take any value)
+      const int whole = max(0, min(r.L, r.L - r.ql + x.rt * p.tok + 1));
+      const uint32_t g_end = g0 + (x.hi - x.kt);
+      volatile float* top_now = xm + (x.piece & 1) * 128 + row;
+      float m = -INFINITY;                                // the running maximum as this thread knows it
+      unsigned long long l2 = 0;                          // two partial sums
+      bool any_tile = false;
+      for (; g < g_end; g += SETS, ++turn) {
+        const int key = (x.kt + (int)(g - g0)) * kKeys;
+        const bool head = g == g0;
+        ok = all_wait(s_bar, turn);
         if (!ok) break;
+        tc_fence_after();
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        uint32_t s0[32];
+        auto load = [&](int c) {                          // 32 scores
+          tm_ld32(s0, s_addr + 32 * c);
+          tm_wait_ld();
+          tm_ready(s0);
+          if (key + 32 * c + 32 > whole) {
+            const int rel = lim - key - 32 * c;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i >= rel) s0[i] = 0xff800000u;
+          }
+        };
+        // (rolled loops, and no register to spare: unrolled, the code of all roles leaves the instruction cache, and a
+        // spilled register costs an L2 access, since the L1 cache is all shared memory; each made the launch 8 to 15 % longer)
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          load(c);
+#pragma unroll
+          for (int i = 0; i < 32; i += 2)
+            mx[i / 2 & 3] = fmaxf(mx[i / 2 & 3], fmaxf(__uint_as_float(s0[i]), __uint_as_float(s0[i + 1])));
+        }
+        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.c;
+        // (also at the head of a piece: no barrier may get two phases ahead of its reader)
+        if (g > 0) ok = all_wait(word_before, (g - 1) / SETS);
+        if (!ok) break;
+        const float m_old = m, m_in = head ? -INFINITY : *top_now;
+        const bool move = top > m_in + kMaxLag;
+        m = move ? (top == INFINITY ? 0.0f : top) : m_in;
+        if (move || head) *top_now = m;
+        mbar_arrive_u32(my_word);
+        if (__any_sync(0xffffffffu, m != m_old)) {
+          const float al = m == m_old ? 1.0f : fast_exp2(m_old - m);
+          l2 = mul2(l2, pack2(al, al));
+          if (!head && __any_sync(0xffffffffu, move)) {
+            // the output of the tiles before this one, all of whose value products must have been added first
+            ok = all_wait(o_done0 + 8 * before, (g - 1) / SETS);
+            if (!ok) break;
+            tc_fence_after();
+            const float al_o = move ? fast_exp2(m_in - m) : 1.0f;
+#pragma unroll 1
+            for (int i = 0; i < D; i += 16) {
+              uint32_t o[16];
+              tm_ld16(o, lane_base + S::OCOL + i);
+              tm_wait_ld();
+              tm_ready16(o);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * al_o);
+              tm_st16(lane_base + S::OCOL + i, o);
+            }
+          }
+        }
+        const float mu = m == -INFINITY ? 0.0f : -m;
+        const unsigned long long c2 = pack2(p.c, p.c), m2 = pack2(mu, mu);
+        // from the last 32 scores (still in registers) to the first, so that the probabilities of a part, 16 columns, go over
+        // scores that have been read: columns 64 .. 127 in the end
+#pragma unroll 1
+        for (int c = 3;; --c) {
+          uint32_t ph16[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            float a, b;
+            unpack2(fma2(pack2(__uint_as_float(s0[2 * k]), __uint_as_float(s0[2 * k + 1])), c2, m2), a, b);
+            a = fast_exp2(a);
+            b = fast_exp2(b);
+            l2 = add2(l2, pack2(a, b));
+            ph16[k] = pack_f16x2(a, b);
+          }
+          tm_st16(s_addr + 64 + 16 * c, ph16);
+          if (c == 0) break;
+          load(c - 1);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        mbar_arrive_u32(p_full0 + 8 * set);
+        any_tile = true;
       }
-      if (!divided && live && p.state_o != nullptr && !finish && (D == 128 || wg == 0)) {
-        p.state_ml[2 * st_row] = m;
-        p.state_ml[2 * st_row + 1] = l;
+      if (!ok) break;
+      // the set's sum under the piece's last maximum, for the end warps, which have read those of the piece before
+      float l = 0.0f, l_hi;
+      if (any_tile) {
+        unpack2(l2, l, l_hi);
+        l += l_hi;
+        if (g_end > g - SETS + 1) {                       // another set has the last tile
+          const uint32_t gl = g_end - 1;
+          ok = all_wait(told0 + 8 * (gl % SETS * 4 + quad), gl / SETS);
+          if (!ok) break;
+          const float m_end = *top_now;
+          if (m_end != m) l *= fast_exp2(m - m_end);
+        }
       }
-      tc_fence_before();               // the accumulator has been read: the next piece's first arrival lets it be overwritten
-      first_piece = false;
-      if (cut) break;
+      if (x.piece > 0) ok = all_wait(ml_free, x.piece - 1);
+      if (!ok) break;
+      xl[set * 128 + row] = l;
+      mbar_arrive_u32(ml_full);
+      g0 = g_end;
+      x.next_piece();
     }
   }
   __syncwarp();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  if (warp == SOFT) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
   if (tid == 0 && *abort && p.status != nullptr) atomicExch(p.status, HKV_ERR_DEVICE_WAIT);
 }
 
@@ -860,17 +915,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) attend_kernel(const __grid_cons
 // parts of a divided row tile (and the state of earlier chunks) -> output or state; a thread has eight channels of a row
 template <int D>
 __global__ void __launch_bounds__(256) merge_kernel(const __grid_constant__ PrefillParams p) {
-  using S = PfShape<D>;
   constexpr int LPR = D / 8;
   pdl_wait();
   pdl_launch_dependents();
   const PfSplit sp = p.split[blockIdx.x];
   const PfStart t = p.start[sp.c2];                       // the row tile: the last of its CTAs begins inside it
   const PfReq r = p.req[t.req];
-  const int piece_tok = S::NT * p.tok;
-  const int prow = blockIdx.y * (256 / LPR) + threadIdx.x / LPR, ch = (threadIdx.x % LPR) * 8;
-  const int row = prow & 127, tk = row / p.G;
-  const int token = t.rt * piece_tok + (prow >> 7) * p.tok + tk;
+  const int row = blockIdx.y * (256 / LPR) + threadIdx.x / LPR, ch = (threadIdx.x % LPR) * 8;
+  const int tk = row / p.G, token = t.rt * p.tok + tk;
   if (tk >= p.tok || token >= r.ql) return;               // (a row's lanes agree)
   const int HQ = p.KVH * p.G;
   const long long st_row = (long long)token * HQ + t.h * p.G + (row - tk * p.G);
@@ -891,10 +943,9 @@ __global__ void __launch_bounds__(256) merge_kernel(const __grid_constant__ Pref
   if (state && !p.first_chunk) add(p.state_ml[2 * st_row], p.state_ml[2 * st_row + 1], p.state_o + st_row * D + ch);
   for (int c = sp.c1; c <= sp.c2; ++c) {
     const long long slot = (long long)c * 2 + (c == sp.c1 ? sp.slot1 : 0);
-    add(p.part_ml[slot * 2 * S::ROWS + prow], p.part_ml[(slot * 2 + 1) * S::ROWS + prow],
-        p.part_o + (slot * S::ROWS + prow) * D + ch);
+    add(p.part_ml[slot * 256 + row], p.part_ml[slot * 256 + 128 + row], p.part_o + (slot * 128 + row) * D + ch);
   }
-  const int end = (max(1, min(r.L, r.L - r.ql + min(r.ql, (t.rt + 1) * piece_tok))) + kKeys - 1) / kKeys;
+  const int end = (max(1, min(r.L, r.L - r.ql + min(r.ql, (t.rt + 1) * p.tok))) + kKeys - 1) / kKeys;
   if (state && end > p.kt_hi) {
     float* so = p.state_o + st_row * D + ch;
     __syncwarp(__activemask());                           // a row's lanes have read its state
@@ -916,15 +967,15 @@ __global__ void __launch_bounds__(256) merge_kernel(const __grid_constant__ Pref
 // ---------------------------------------------------------------------------------------------------------- the plan
 // Cuts the key tiles of the launch into at most n_cta shares of equal cost; returns the CTAs used. Greedy: a CTA takes
 // row tiles in order until its share is full, and divides the one that does not fit when both parts are long enough.
-static int plan(PrefillParams& p, int piece_tok, int n_cta, int* n_split) {
+static int plan(PrefillParams& p, int n_cta, int* n_split) {
   long long total = 0;
   Walk w0{0, 0, -1, 0};
-  w0.advance(p.req, p.n_req, p.KVH, piece_tok, p.kt_lo, p.kt_hi);      // the first row tile with keys in the chunk
+  w0.advance(p.req, p.n_req, p.KVH, p.tok, p.kt_lo, p.kt_hi);      // the first row tile with keys in the chunk
   for (int r = 0; r < p.n_req; ++r) {
     long long head = 0;
-    const int n_rt = pf_row_tiles(p.req[r], piece_tok);
+    const int n_rt = pf_row_tiles(p.req[r], p.tok);
     for (int rt = 0; rt < n_rt; ++rt) {
-      const int n = pf_hi(p.req[r], rt, piece_tok, p.kt_hi) - p.kt_lo;
+      const int n = pf_hi(p.req[r], rt, p.tok, p.kt_hi) - p.kt_lo;
       if (n > 0) head += kPieceCost + n;
     }
     total += head * p.KVH;
@@ -941,7 +992,7 @@ static int plan(PrefillParams& p, int piece_tok, int n_cta, int* n_split) {
     auto begin = [&]() { p.start[c] = PfStart{w.kt, w.rt, (short)w.h, (short)w.req}; room = cap; pieces = 0; };
     if (w.req < p.n_req) begin();
     while (w.req < p.n_req) {
-      const int hi = pf_hi(p.req[w.req], w.rt, piece_tok, p.kt_hi);
+      const int hi = pf_hi(p.req[w.req], w.rt, p.tok, p.kt_hi);
       const int n = hi - w.kt;
       if (kPieceCost + n <= room) {                       // the rest of the row tile
         if (part_c1 >= 0) {
@@ -950,7 +1001,7 @@ static int plan(PrefillParams& p, int piece_tok, int n_cta, int* n_split) {
         }
         room -= kPieceCost + n;
         ++pieces;
-        w.advance(p.req, p.n_req, p.KVH, piece_tok, p.kt_lo, p.kt_hi);
+        w.advance(p.req, p.n_req, p.KVH, p.tok, p.kt_lo, p.kt_hi);
         if (w.req >= p.n_req) break;
         continue;
       }
@@ -1016,12 +1067,12 @@ static PfScratch prefill_scratch(const int32_t* rows, int n_rows, int n_tok, int
     }
     i += g.n;
   }
-  const size_t rws = D == 128 ? 256 : 128, n_cta = prefill_ctas();
+  const size_t n_cta = prefill_ctas();
   PfScratch s;
   s.tiles = 0;
   s.part_o = a256(s.tiles + (size_t)max_tiles * KVH * 2 * kKeys * D * 2);
-  s.part_ml = a256(s.part_o + n_cta * 2 * rws * D * 4);
-  s.state_o = a256(s.part_ml + n_cta * 2 * 2 * rws * 4);
+  s.part_ml = a256(s.part_o + n_cta * 2 * 128 * D * 4);
+  s.state_o = a256(s.part_ml + n_cta * 2 * 2 * 128 * 4);
   s.state_ml = a256(s.state_o + state_rows * D * 4);
   s.rot = a256(s.state_ml + state_rows * 8);
   s.total = a256(s.rot + (rot ? (size_t)n_tok * KVH * G * D * 2 : 0));
@@ -1053,10 +1104,10 @@ extern "C" size_t hkv_prefill_scratch_bytes(const int32_t* rows, int n_rows, int
   return prefill_scratch(rows, n_rows, n_tokens, KVH, G, D, chunk_tiles_of(chunk), rotated).total;
 }
 
-extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const void* ksf, const void* vd, const void* vsf,
+extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
                            const int64_t strides[6], int PS, const int32_t* block_tables, int n_tables, int MP,
                            const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale,
-                           int k_f16, const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out,
+                           const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out,
                            int out_f32, void* workspace, void* stream) {
   using namespace hkv;
   if (n_rows == 0) return HKV_OK;
@@ -1065,7 +1116,7 @@ extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const voi
   if (rc != HKV_OK) return rc;
   if (k8 && D != 256) return HKV_ERR_UNSUPPORTED;
   if (!q || !kd || !ksf || !vd || !vsf || !strides || !block_tables || !scratch || !out) return HKV_ERR_NULL;
-  if (signs && (k8 || q_ready)) return HKV_ERR_UNSUPPORTED;
+  if (signs && (k8 || q_f16)) return HKV_ERR_UNSUPPORTED;
   if (PS < 1) return HKV_ERR_UNSUPPORTED;
   if (((uintptr_t)kd | (uintptr_t)vd | (uintptr_t)strides[0] | (uintptr_t)strides[1] | (uintptr_t)strides[2]) & 7) return HKV_ERR_ALIGN;
   if (k8 && (((uintptr_t)kd | (uintptr_t)strides[0] | (uintptr_t)strides[1] | (uintptr_t)strides[2]) & 15)) return HKV_ERR_ALIGN;
@@ -1080,24 +1131,21 @@ extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const voi
 
   PrefillParams p = {};
   p.q = q;
-  p.q_cvt = k_f16 && !q_ready;
   if (signs) {
     const long long n = (long long)n_tokens * KVH * G;
     const float scale = (float)(1.0 / sqrt((double)D));
-    void (*k)(const __nv_bfloat16*, const float*, uint32_t*, long long, float, int) = D == 128 ? rotate_kernel<128> : rotate_kernel<256>;
+    void (*k)(const __nv_bfloat16*, const float*, uint32_t*, long long, float) = D == 128 ? rotate_kernel<128> : rotate_kernel<256>;
     rc = record_cuda(launch_pdl(k, dim3((unsigned)((n + 7) / 8)), dim3(256), 0, st, (const __nv_bfloat16*)q, signs,
-                                (uint32_t*)(base + sc.rot), n, scale, k_f16 ? 0 : 1));
+                                (uint32_t*)(base + sc.rot), n, scale));
     if (rc != HKV_OK) return rc;
     p.q = base + sc.rot;
-    p.q_cvt = 0;
   }
   const float c = qk_scale * 1.4426950408889634f;
-  p.q_flip = c < 0.0f ? 0x80008000u : 0u;
   p.c = fmaxf(fabsf(c), 1e-37f);                          // (zero: masked scores would become 0 * -inf)
   p.vs = out_scale;
   p.out = out;
   p.out_f32 = out_f32;
-  p.k_bf16 = !k_f16;
+  p.k_bf16 = !q_f16;                                      // (the cached values are exact in both types)
   p.KVH = KVH;
   p.G = G;
   p.tok = 128 / G;
@@ -1105,7 +1153,7 @@ extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const voi
   p.part_o = (float*)(base + sc.part_o);
   p.part_ml = (float*)(base + sc.part_ml);
   p.status = workspace ? &((Header*)workspace)->status : nullptr;
-  const int piece_tok = (D == 128 ? 2 : 1) * p.tok, n_cta = prefill_ctas();
+  const int n_cta = prefill_ctas();
 
   TileParams t = {};
   t.kd = (const uint8_t*)kd; t.ksf = (const uint8_t*)ksf; t.vd = (const uint8_t*)vd; t.vsf = (const uint8_t*)vsf;
@@ -1113,10 +1161,11 @@ extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const voi
   t.ssp = strides[3]; t.sst = strides[4]; t.ssh = strides[5];
   t.bt = block_tables; t.tiles = base + sc.tiles;
   t.MP = MP; t.PS = PS; t.KVH = KVH;
+  t.k_flip = c < 0.0f ? 0x80008000u : 0u;
   void (*tk)(const TileParams);
-  if (k8) tk = k_f16 ? tile_kernel<256, 0, 1> : tile_kernel<256, 1, 1>;
-  else if (D == 128) tk = k_f16 ? tile_kernel<128, 0, 0> : tile_kernel<128, 1, 0>;
-  else tk = k_f16 ? tile_kernel<256, 0, 0> : tile_kernel<256, 1, 0>;
+  if (k8) tk = q_f16 ? tile_kernel<256, 0, 1> : tile_kernel<256, 1, 1>;
+  else if (D == 128) tk = q_f16 ? tile_kernel<128, 0, 0> : tile_kernel<128, 1, 0>;
+  else tk = q_f16 ? tile_kernel<256, 0, 0> : tile_kernel<256, 1, 0>;
   void (*ak)(const PrefillParams) = D == 128 ? attend_kernel<128> : attend_kernel<256>;
   void (*mk)(const PrefillParams) = D == 128 ? merge_kernel<128> : merge_kernel<256>;
   rc = record_cuda(cudaFuncSetAttribute((const void*)ak, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
@@ -1144,11 +1193,11 @@ extern "C" int hkv_prefill(const void* q, int q_ready, const void* kd, const voi
       p.kt_hi = g.chunked ? (lo + ct < all_tiles ? lo + ct : all_tiles) : all_tiles;
       t.n_tiles = g.chunked ? p.kt_hi - lo : base_tile;
       int n_split = 0;
-      const int used = plan(p, piece_tok, n_cta, &n_split);
+      const int used = plan(p, n_cta, &n_split);
       rc = record_cuda(launch_pdl(tk, dim3((unsigned)t.n_tiles, (unsigned)KVH, 2), dim3(128), 0, st, t));
-      if (rc == HKV_OK) rc = record_cuda(launch_pdl(ak, dim3((unsigned)used), dim3(kPfThreads), kPfSmem, st, p));
+      if (rc == HKV_OK) rc = record_cuda(launch_pdl(ak, dim3((unsigned)used), dim3(D == 128 ? PfShape<128>::THREADS : PfShape<256>::THREADS), kPfSmem, st, p));
       if (rc == HKV_OK && n_split > 0)
-        rc = record_cuda(launch_pdl(mk, dim3((unsigned)n_split, 16), dim3(256), 0, st, p));
+        rc = record_cuda(launch_pdl(mk, dim3((unsigned)n_split, D == 128 ? 8 : 16), dim3(256), 0, st, p));
       if (rc != HKV_OK) return rc;
       if (!g.chunked) break;
     }

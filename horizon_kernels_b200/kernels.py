@@ -247,26 +247,25 @@ def dequant_multi(flat, strides, PS, block_tables, rows, cu, n_rows, n_tokens, o
     _dequant(flat, strides, PS, block_tables, block_tables.shape[1], rows, cu, n_rows, 0, n_tokens, out_k, out_v, k8)
 
 
-def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out, chunk=65536, k_f16=True,
-            signs=None, k8=False, workspace=None):
+def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out, chunk=65536, signs=None,
+            k8=False, workspace=None):
     """rows: [(table row, q0, q1, L)] with q0 < q1 and L >= 1: query tokens q0 .. q1 - 1 against the first L cached
-    tokens of block_tables[row], query token t of ql seeing keys j < L - ql + t + 1. query (NT, HQ, D) bf16 contiguous,
-    or already in the compute type (fp16 with k_f16); out (>= NT, HQ, D) bf16 or fp32 contiguous, other rows untouched.
+    tokens of block_tables[row], query token t of ql seeing keys j < L - ql + t + 1. query (NT, HQ, D) bf16 or fp16
+    contiguous; out (>= NT, HQ, D) bf16 or fp32 contiguous, other rows untouched.
     out = softmax(q k^T * qk_scale) v * out_scale, the cached values taken without their global scales. `chunk` bounds
     the tokens that are held as 16-bit operands at a time; the scratch comes from torch's allocator. signs as in
     decode_ragged. The reference's counterpart is backend.py:438-543."""
     rc = (_lib._host or _lib.host()).prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out,
-                                             chunk, k_f16, signs, k8, workspace)
+                                             chunk, signs, k8, workspace)
     if rc is not None:
         if rc:
             _lib.check(rc, "hkv_prefill")
         return out
     if k8 and signs is not None:
         raise ValueError("the K8V4 slot keeps FP8 keys: no rotation")
-    ready = query.dtype == torch.float16
-    if query.dtype != torch.bfloat16 and not (ready and k_f16):
-        raise TypeError("query must be bf16, or fp16 with fp16 compute")
-    if ready and signs is not None:
+    if query.dtype not in (torch.bfloat16, torch.float16):
+        raise TypeError("query must be bf16 or fp16")
+    if query.dtype == torch.float16 and signs is not None:
         raise TypeError("query to be rotated must be bf16")
     if out.dtype not in (torch.bfloat16, torch.float32):
         raise TypeError("out must be bf16 or fp32")
@@ -294,9 +293,9 @@ def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, K
     kd, ksf, vd, vsf = flat
     with torch.cuda.device(query.device):
         scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device=query.device)
-        rc = lib.hkv_prefill(_ptr(query), int(signs is None and (ready or not k_f16)), _ptr(kd), _ptr(ksf), _ptr(vd), _ptr(vsf),
+        rc = lib.hkv_prefill(_ptr(query), int(query.dtype == torch.float16), _ptr(kd), _ptr(ksf), _ptr(vd), _ptr(vsf),
                              (C.c_int64 * 6)(*strides), int(PS), _ptr(block_tables), B, MP, host_rows, n, NT, KVH, HQ // KVH,
-                             D, float(qk_scale), float(out_scale), int(bool(k_f16)), None if signs is None else _ptr(signs),
+                             D, float(qk_scale), float(out_scale), None if signs is None else _ptr(signs),
                              int(bool(k8)), int(chunk), _ptr(scratch), nb, _ptr(out), int(out.dtype == torch.float32),
                              None if workspace is None else _ptr(workspace), _stream())
     _lib.check(rc, "hkv_prefill")

@@ -224,14 +224,13 @@ int hkv_selftest_wait_timeout(void* workspace, int64_t cycles, void* stream);
 /*
  * Prefill attention: rows of requests with many query tokens against their cached context (the new tokens included; call
  * hkv_write first), causal. Replaces the reference's dequantisation + library attention (backend.py:438-543).
- *   q               (n_tokens, KVH * G, D) 16 bits, contiguous, 16-byte aligned: bf16, or (q_ready) already in the
- *                   compute type: f16 with k_f16, bf16 without
+ *   q               (n_tokens, KVH * G, D), contiguous, 16-byte aligned, bf16 or (q_f16) f16: also the type of the score
+ *                   product's operands (the cached values without their global scale are exact in both). Probabilities
+ *                   and values are f16, all sums fp32.
  *   kd .. MP        the cache and the block tables (n_tables, MP) int32, as for hkv_decode
  *   rows            HOST array of n_rows x {table row, first query token, one past the last, context length}: query token
  *                   t of ql sees the keys j < L - ql + t + 1. It is read before the call returns.
- *   k_f16           type of the score product's operands: f16 (nonzero) or bf16; the cached values are exact in both.
- *                   Probabilities and values are f16, all sums fp32.
- *   signs           as hkv_decode_rot (q is rotated in fp32 on the way to the compute type), or NULL; not with k8 / q_ready
+ *   signs           as hkv_decode_rot, or NULL; not with k8 or q_f16
  *   k8              K8V4 slot: kd = key bytes, ksf unused but not NULL
  *   chunk           cached tokens held as 16-bit operands at a time (at least 128); longer contexts are attended chunk by
  *                   chunk with an fp32 state
@@ -244,9 +243,9 @@ int hkv_selftest_wait_timeout(void* workspace, int64_t cycles, void* stream);
  */
 size_t hkv_prefill_scratch_bytes(const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, int64_t chunk,
                                  int rotated);
-int hkv_prefill(const void* q, int q_ready, const void* kd, const void* ksf, const void* vd, const void* vsf,
+int hkv_prefill(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
                 const int64_t strides[6], int PS, const int32_t* block_tables, int n_tables, int MP, const int32_t* rows,
-                int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale, int k_f16,
+                int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale,
                 const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out, int out_f32,
                 void* workspace, void* stream);
 

@@ -14,7 +14,7 @@ from oracle import kvfp4 as O
 pytestmark = pytest.mark.gpu
 
 
-def run_case(qls, lens, KVH, G, D, PS=16, chunk=65536, k_f16=True, out_dtype=torch.bfloat16, seed=5, qk_scale=None):
+def run_case(qls, lens, KVH, G, D, PS=16, chunk=65536, q_dtype=torch.bfloat16, out_dtype=torch.bfloat16, seed=5, qk_scale=None):
     c = synth.paged_case(seed + D, lens, KVH, G, D, PS, outliers=True, ql_list=qls)
     dev = torch.device("cuda")
     gk = torch.full((KVH,), 0.04, device=dev)
@@ -22,7 +22,7 @@ def run_case(qls, lens, KVH, G, D, PS=16, chunk=65536, k_f16=True, out_dtype=tor
     cache = Lt.alloc_cache(c["NP"], PS, KVH, D, device=dev, fill=0x7F)
     flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
     K.write(bf16_tensor(c["key"]), bf16_tensor(c["val"]), flat, strides, PS, torch.from_numpy(c["slots"]).to(dev), gk, gv)
-    q = bf16_tensor(c["q"])
+    q = bf16_tensor(c["q"]).to(q_dtype)                  # (exact: the values are ordinary)
     NT = q.shape[0]
     out = torch.full((NT + 3, KVH * G, D), 5.0, dtype=out_dtype, device=dev)
     qsl = [int(x) for x in c["qsl"]]
@@ -30,7 +30,7 @@ def run_case(qls, lens, KVH, G, D, PS=16, chunk=65536, k_f16=True, out_dtype=tor
     sm = D ** -0.5 if qk_scale is None else qk_scale
     ws = K.alloc_workspace(4, KVH, min(G, 8), D)
     K.prefill(q, flat, strides, PS, torch.from_numpy(c["bt"]).to(dev), rows, sm * 0.04, 1.0, KVH, out, chunk=chunk,
-              k_f16=k_f16, workspace=ws)
+              workspace=ws)
     assert K.workspace_status(ws) == 0
     assert (out[NT:] == 5.0).all()
     lay = O.Layout.slots(PS, KVH, D)
@@ -73,8 +73,8 @@ def test_divided_row_tiles(D):
     run_case([3], [20000], 1, 4, D)
 
 
-def test_bf16_scores():
-    run_case([100], [500], 2, 4, 128, k_f16=False)
+def test_fp16_queries():
+    run_case([100], [500], 2, 4, 128, q_dtype=torch.float16)
 
 
 @pytest.mark.parametrize("D", [128, 256])
