@@ -90,15 +90,22 @@ struct Geo {
   __device__ static constexpr int kblk(int c, int u) { return NBL * c + u; }
 };
 
-// QT: 8-row query tiles of one pass (1, or 2 at head_dim 128: sixteen query rows per kv head read the cache once)
+// QT: 8-row query tiles of one pass (1, or 2: sixteen query rows per kv head read the cache once). At head_dim 256 the two
+// tiles' accumulators take 128 registers: the query fragments lie in shared memory (QSM), where a piece's merge buffer lies
+// afterwards, a unit's two 16-token blocks are worked on one after the other and the merge takes one tile at a time, so that
+// two CTAs still fit an SM (245 registers, none spilled). 96 requests of 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query
+// tokens, rotated keys: 102 us in one pass against 146 in two of eight rows. (At head_dim 128 the fragments stay in registers:
+// the same layout there lets a third CTA in, and took 62 to 67 us where this one takes 59.)
 template <int D, int LAYOUT, int QT = 1>
 struct Smem {
   using G_ = Geo<D, LAYOUT>;
   static constexpr int RP = RPAD * QT;                              // query rows of one pass
+  static constexpr bool QSM = D == 256 && QT == 2;
+  static constexpr int MP = QSM ? QT : 1;                           // passes of a piece's merge
   static constexpr int RING = TG * G_::NS * G_::STAGE;
   static constexpr int BARS = TG * G_::NS * 8;
   static constexpr int OROW = D + 4;                               // padded accumulator row (floats)
-  static constexpr int MERGE = TG * RP * OROW * 4 + TG * RP * 2 * 4;
+  static constexpr int MERGE = TG * (RP / MP) * OROW * 4 + TG * RP * 2 * 4;
   static constexpr int COARSE = (kMaxBatch / 32 + 2) * 4;
   static constexpr int TOTAL = RING + BARS + MERGE + COARSE + 64;
 };
@@ -109,11 +116,12 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
   using Sm = Smem<D, LAYOUT, QT>;
   constexpr int RP = Sm::RP;
   constexpr int NS = Gm::NS, UB = Gm::UB, UT = Gm::UT, LOG_UT = Gm::LOG_UT;
+  constexpr int BB = Sm::QSM ? 1 : UB;             // 16-token blocks of a unit worked on at a time (registers)
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t* ring = smem;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Sm::RING);
   float* obuf = reinterpret_cast<float*>(smem + Sm::RING + Sm::BARS);
-  float* mbuf = obuf + TG * RP * Sm::OROW;
+  float* mbuf = obuf + TG * (RP / Sm::MP) * Sm::OROW;
   float* lbuf = mbuf + TG * RP;
   int* coarse = reinterpret_cast<int*>(smem + Sm::RING + Sm::BARS + Sm::MERGE);
   __shared__ SplitSeq split[2];
@@ -456,75 +464,90 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       for (int j = 0; j < Gm::KS; ++j) o[q][j][0] = o[q][j][1] = o[q][j][2] = o[q][j][3] = 0.0f;
     }
 
-    if (blk_first < blk_end && !dead) {
-      // softmax scale in the log2 domain. A negative scale is moved into the query so that "max" stays a max.
-      float sc = p.scale_log2 * __ldg(p.gk + h);
-      const bool flip = sc < 0.0f;
-      sc = fmaxf(fabsf(sc), 1e-30f);
-      const float tau_raw = TAU / sc;
-      // query fragments: row g of the (request, kv head) group, channels of this lane's key blocks, as f16
-      uint32_t qa[QT][Gm::KS][2];
+    // query fragments: row g (+ 8 q) of the (request, kv head) group, channels of this lane's key blocks, as f16
+    auto load_queries = [&](int q, bool flip, uint32_t (&out)[Gm::KS][2]) {
+      const bool have = g + 8 * q < R;
+      const int t = have ? (p.row0 + g + 8 * q) / G : 0, gq = have ? p.row0 + g + 8 * q - t * G : 0;
+      const __nv_bfloat16* qrow = p.q + ((long long)(q0 + t) * (KVH * G) + h * G + gq) * D;
+      constexpr int NQ = 16 * Gm::NBL;            // this lane's channels: NQ * c .. NQ * c + NQ - 1 of the row
+      float qf[NQ];
 #pragma unroll
-      for (int q = 0; q < QT; ++q) {
-        const bool have = g + 8 * q < R;
-        const int t = have ? (p.row0 + g + 8 * q) / G : 0, gq = have ? p.row0 + g + 8 * q - t * G : 0;
-        const __nv_bfloat16* qrow = p.q + ((long long)(q0 + t) * (KVH * G) + h * G + gq) * D;
-        constexpr int NQ = 16 * Gm::NBL;            // this lane's channels: NQ * c .. NQ * c + NQ - 1 of the row
-        float qf[NQ];
-#pragma unroll
-        for (int u = 0; u < Gm::NBL; ++u) {
-          uint4 x0 = make_uint4(0, 0, 0, 0), x1 = make_uint4(0, 0, 0, 0);
-          if (have) {
-            const uint4* src = reinterpret_cast<const uint4*>(qrow + 16 * Gm::kblk(c, u));
-            x0 = __ldg(src);
-            x1 = __ldg(src + 1);
-          }
-          const uint32_t ws[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            qf[16 * u + 2 * i] = __uint_as_float(ws[i] << 16);
-            qf[16 * u + 2 * i + 1] = __uint_as_float(ws[i] & 0xffff0000u);
-          }
+      for (int u = 0; u < Gm::NBL; ++u) {
+        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = make_uint4(0, 0, 0, 0);
+        if (have) {
+          const uint4* src = reinterpret_cast<const uint4*>(qrow + 16 * Gm::kblk(c, u));
+          x0 = __ldg(src);
+          x1 = __ldg(src + 1);
         }
-        if (p.signs != nullptr) {
-          // keys were written rotated: q' = bf16(FWHT(q * signs) * head_dim^-0.5), the reference's rotate_q
-          // (kv_fp4_ref.py:90-92), fp32 butterflies in its stage order. The four lanes of a quad hold one row.
-          const float4* sg = reinterpret_cast<const float4*>(p.signs + NQ * c);
+        const uint32_t ws[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-          for (int i = 0; i < NQ / 4; ++i) {
-            const float4 s4 = __ldg(sg + i);
-            qf[4 * i] = __fmul_rn(qf[4 * i], s4.x);
-            qf[4 * i + 1] = __fmul_rn(qf[4 * i + 1], s4.y);
-            qf[4 * i + 2] = __fmul_rn(qf[4 * i + 2], s4.z);
-            qf[4 * i + 3] = __fmul_rn(qf[4 * i + 3], s4.w);
-          }
+        for (int i = 0; i < 8; ++i) {
+          qf[16 * u + 2 * i] = __uint_as_float(ws[i] << 16);
+          qf[16 * u + 2 * i + 1] = __uint_as_float(ws[i] & 0xffff0000u);
+        }
+      }
+      if (p.signs != nullptr) {
+        // keys were written rotated: q' = bf16(FWHT(q * signs) * head_dim^-0.5), the reference's rotate_q
+        // (kv_fp4_ref.py:90-92), fp32 butterflies in its stage order. The four lanes of a quad hold one row.
+        const float4* sg = reinterpret_cast<const float4*>(p.signs + NQ * c);
 #pragma unroll
-          for (int hh = 1; hh < NQ; hh *= 2)
+        for (int i = 0; i < NQ / 4; ++i) {
+          const float4 s4 = __ldg(sg + i);
+          qf[4 * i] = __fmul_rn(qf[4 * i], s4.x);
+          qf[4 * i + 1] = __fmul_rn(qf[4 * i + 1], s4.y);
+          qf[4 * i + 2] = __fmul_rn(qf[4 * i + 2], s4.z);
+          qf[4 * i + 3] = __fmul_rn(qf[4 * i + 3], s4.w);
+        }
 #pragma unroll
-            for (int i = 0; i < NQ; ++i)
-              if ((i & hh) == 0) {
-                const float a = qf[i], b = qf[i + hh];
-                qf[i] = __fadd_rn(a, b);
-                qf[i + hh] = __fsub_rn(a, b);
-              }
+        for (int hh = 1; hh < NQ; hh *= 2)
 #pragma unroll
-          for (int m = 1; m < 4; m *= 2) {          // stages h = NQ, 2 NQ: the partner is the lane with c ^ m
-            const bool upper = (c & m) != 0;
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) {
-              const float o2 = __shfl_xor_sync(0xffffffffu, qf[i], m);
-              qf[i] = upper ? __fsub_rn(o2, qf[i]) : __fadd_rn(qf[i], o2);
+          for (int i = 0; i < NQ; ++i)
+            if ((i & hh) == 0) {
+              const float a = qf[i], b = qf[i + hh];
+              qf[i] = __fadd_rn(a, b);
+              qf[i + hh] = __fsub_rn(a, b);
             }
+#pragma unroll
+        for (int m = 1; m < 4; m *= 2) {          // stages h = NQ, 2 NQ: the partner is the lane with c ^ m
+          const bool upper = (c & m) != 0;
+#pragma unroll
+          for (int i = 0; i < NQ; ++i) {
+            const float o2 = __shfl_xor_sync(0xffffffffu, qf[i], m);
+            qf[i] = upper ? __fsub_rn(o2, qf[i]) : __fadd_rn(qf[i], o2);
           }
-#pragma unroll
-          for (int i = 0; i < NQ; ++i) qf[i] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(qf[i], p.rot_scale)));
         }
 #pragma unroll
-        for (int i = 0; i < NQ / 2; ++i) {
-          float a = qf[2 * i], bq = qf[2 * i + 1];
-          if (flip) { a = -a; bq = -bq; }
-          qa[q][i >> 1][i & 1] = pack_f16x2_sat(a, bq);   // values beyond f16's range become +-65504
-        }
+        for (int i = 0; i < NQ; ++i) qf[i] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(qf[i], p.rot_scale)));
+      }
+#pragma unroll
+      for (int i = 0; i < NQ / 2; ++i) {
+        float a = qf[2 * i], bq = qf[2 * i + 1];
+        if (flip) { a = -a; bq = -bq; }
+        out[i >> 1][i & 1] = pack_f16x2_sat(a, bq);   // values beyond f16's range become +-65504
+      }
+    };
+    // softmax scale in the log2 domain. A negative scale is moved into the query so that "max" stays a max.
+    const float sc_signed = p.scale_log2 * __ldg(p.gk + h);
+    const bool flip = sc_signed < 0.0f;
+    const uint32_t qs_a = smem_u32(obuf) + lane * 8;       // (QSM) this lane's fragment of k-step s of tile q: + (q * KS + s) * 256
+    if constexpr (Sm::QSM) {
+      if (w < QT) {
+        uint32_t f[Gm::KS][2];
+        load_queries(w, flip, f);
+#pragma unroll
+        for (int k = 0; k < Gm::KS; ++k)
+          asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(qs_a + (w * Gm::KS + k) * 256), "r"(f[k][0]), "r"(f[k][1]) : "memory");
+      }
+      __syncthreads();
+    }
+
+    if (blk_first < blk_end && !dead) {
+      const float sc = fmaxf(fabsf(sc_signed), 1e-30f);
+      const float tau_raw = TAU / sc;
+      uint32_t qa[Sm::QSM ? 1 : QT][Gm::KS][2];
+      if constexpr (!Sm::QSM) {
+#pragma unroll
+        for (int q = 0; q < QT; ++q) load_queries(q, flip, qa[q]);
       }
       // visible context of query rows 2c, 2c+1 (causal among the request's own query tokens)
       int lim0[QT], lim1[QT];
@@ -559,10 +582,17 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       };
 
       // ---------------- S^T = K Q^T per 16-token block: rows = tokens, columns = query rows
-      auto k_phase = [&](const uint32_t st, float (&x)[QT][UB][4]) {
-        const uint32_t kd_ = st + koff_d, ks_ = st + koff_s;
+      auto score_mma = [&](float (&d)[4], const uint32_t (&a)[4], int q, int step) {
+        uint2 b;
+        if constexpr (Sm::QSM) b = lds64(qs_a + (q * Gm::KS + step) * 256);
+        else b = make_uint2(qa[q][step][0], qa[q][step][1]);
+        mma_f16(d, a[0], a[1], a[2], a[3], b.x, b.y);
+      };
+      // (bb: first of the BB blocks worked on)
+      auto k_phase = [&](const uint32_t st, const int bb, float (&x)[QT][BB][4]) {
+        const uint32_t kd_ = st + koff_d + bb * 16 * Gm::ROW, ks_ = st + koff_s + bb * 16 * Gm::SF_ROW;
 #pragma unroll
-        for (int bi = 0; bi < UB; ++bi) {
+        for (int bi = 0; bi < BB; ++bi) {
           float sa[QT][Gm::NCH][4];
 #pragma unroll
           for (int q = 0; q < QT; ++q)
@@ -577,12 +607,11 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
               const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
               for (int v = 0; v < 4; ++v) {           // k-step v of the block: channels 4v .. 4v+3 of rows r0, r1
-                uint32_t a0, a2, a1, a3;
-                e4m3x4_to_f16x2(wa[v], a0, a2);
-                e4m3x4_to_f16x2(wb[v], a1, a3);
+                uint32_t A[4];
+                e4m3x4_to_f16x2(wa[v], A[0], A[2]);
+                e4m3x4_to_f16x2(wb[v], A[1], A[3]);
 #pragma unroll
-                for (int q = 0; q < QT; ++q)
-                  mma_f16(sa[q][v & (Gm::NCH - 1)], a0, a1, a2, a3, qa[q][4 * u + v][0], qa[q][4 * u + v][1]);
+                for (int q = 0; q < QT; ++q) score_mma(sa[q][v & (Gm::NCH - 1)], A, q, 4 * u + v);
               }
             }
 #pragma unroll
@@ -632,10 +661,10 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
             const uint32_t A3[4] = {hmul2h(e1[2], sf0), hmul2h(e3[2], sf1), hmul2h(e1[3], sf0), hmul2h(e3[3], sf1)};
 #pragma unroll
             for (int q = 0; q < QT; ++q) {
-              mma_f16(sa[q][0], A0[0], A0[1], A0[2], A0[3], qa[q][4 * u + 0][0], qa[q][4 * u + 0][1]);
-              mma_f16(sa[q][Gm::NCH - 1], A1[0], A1[1], A1[2], A1[3], qa[q][4 * u + 1][0], qa[q][4 * u + 1][1]);
-              mma_f16(sa[q][0], A2[0], A2[1], A2[2], A2[3], qa[q][4 * u + 2][0], qa[q][4 * u + 2][1]);
-              mma_f16(sa[q][Gm::NCH - 1], A3[0], A3[1], A3[2], A3[3], qa[q][4 * u + 3][0], qa[q][4 * u + 3][1]);
+              score_mma(sa[q][0], A0, q, 4 * u);
+              score_mma(sa[q][Gm::NCH - 1], A1, q, 4 * u + 1);
+              score_mma(sa[q][0], A2, q, 4 * u + 2);
+              score_mma(sa[q][Gm::NCH - 1], A3, q, 4 * u + 3);
             }
           }
 #pragma unroll
@@ -648,12 +677,12 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       // ---------------- online softmax (raw score units): this lane holds query rows 2c, 2c+1 of tokens r0, r1 of
       // every block; x[bi] = {(r0, row 2c), (r0, row 2c+1), (r1, row 2c), (r1, row 2c+1)}. Leaves P^T as the B
       // operand of the second product in pb.
-      auto softmax = [&](const uint32_t st, const int blk, float (&x)[QT][UB][4], uint32_t (&pb)[QT][UB][2]) {
+      auto softmax = [&](const uint32_t st, const int blk, const int bb, float (&x)[QT][BB][4], uint32_t (&pb)[QT][BB][2]) {
         const int tbase = blk * UT;
         if (blk >= blk_mask) {                        // warp-uniform: only the last unit(s) of a sequence
           // rows past the context hold arbitrary bytes: their scores become -inf below, and their value scales are
           // set to zero here, in shared memory, so that the value product needs no masking code
-          if (lane < UT && tbase + lane >= L) {
+          if (bb == 0 && lane < UT && tbase + lane >= L) {
             const uint32_t a = st + Gm::V_BASE + Gm::SF_BASE + lane * Gm::SF_ROW;
 #pragma unroll
             for (int i = 0; i < Gm::SS; i += 8) sts64_zero(a + i);
@@ -664,8 +693,8 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
 #pragma unroll
           for (int q = 0; q < QT; ++q)
 #pragma unroll
-            for (int bi = 0; bi < UB; ++bi) {
-              const int ta = tbase + 16 * bi + r0, tb = tbase + 16 * bi + r1;
+            for (int bi = 0; bi < BB; ++bi) {
+              const int ta = tbase + 16 * (bb + bi) + r0, tb = tbase + 16 * (bb + bi) + r1;
               x[q][bi][0] = ta < lim0[q] ? x[q][bi][0] : ninf;
               x[q][bi][1] = ta < lim1[q] ? x[q][bi][1] : ninf;
               x[q][bi][2] = tb < lim0[q] ? x[q][bi][2] : ninf;
@@ -681,7 +710,7 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
           bm0[q] = fmaxf(x[q][0][0], x[q][0][2]);
           bm1[q] = fmaxf(x[q][0][1], x[q][0][3]);
 #pragma unroll
-          for (int bi = 1; bi < UB; ++bi) {
+          for (int bi = 1; bi < BB; ++bi) {
             bm0[q] = fmaxf(bm0[q], fmaxf(x[q][bi][0], x[q][bi][2]));
             bm1[q] = fmaxf(bm1[q], fmaxf(x[q][bi][1], x[q][bi][3]));
           }
@@ -710,7 +739,7 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
 #pragma unroll
         for (int q = 0; q < QT; ++q)
 #pragma unroll
-          for (int bi = 0; bi < UB; ++bi) {
+          for (int bi = 0; bi < BB; ++bi) {
             const float p00 = fast_exp2(fmaf(x[q][bi][0], sc, mneg0[q])), p01 = fast_exp2(fmaf(x[q][bi][1], sc, mneg1[q])),
                         p10 = fast_exp2(fmaf(x[q][bi][2], sc, mneg0[q])), p11 = fast_exp2(fmaf(x[q][bi][3], sc, mneg1[q]));
             l0[q] += p00 + p10;
@@ -722,10 +751,10 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       };
 
       // ---------------- O^T += V^T P^T : rows = channels of block g (+8), columns = query rows
-      auto v_phase = [&](const uint32_t st, const uint32_t (&pb)[QT][UB][2]) {
-        const uint32_t vd_ = st + voff_d, vs_ = st + voff_s;
+      auto v_phase = [&](const uint32_t st, const int bb, const uint32_t (&pb)[QT][BB][2]) {
+        const uint32_t vd_ = st + voff_d + bb * 16 * Gm::ROW, vs_ = st + voff_s + bb * 16 * Gm::SF_ROW;
 #pragma unroll
-        for (int bi = 0; bi < UB; ++bi) {
+        for (int bi = 0; bi < BB; ++bi) {
 #pragma unroll
           for (int hf = 0; hf < Gm::NH; ++hf) {
             const int dv = bi * 16 * Gm::ROW + 64 * hf, sv = bi * 16 * Gm::SF_ROW + 8 * hf;
@@ -769,11 +798,14 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
         }
       } else if (wait_stage(bar, st)) {
         for (int blk = blk_first;;) {
-          float x[QT][UB][4];
-          uint32_t pb[QT][UB][2];
-          k_phase(st, x);
-          softmax(st, blk, x, pb);
-          v_phase(st, pb);
+#pragma unroll 1
+          for (int bb = 0; bb < UB; bb += BB) {
+            float x[QT][BB][4];
+            uint32_t pb[QT][BB][2];
+            k_phase(st, bb, x);
+            softmax(st, blk, bb, x, pb);
+            v_phase(st, bb, pb);
+          }
           __syncwarp();
           if ((int)f_n < n_my) fetch_one(bar, st);
           blk += TG;
@@ -784,72 +816,78 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
 
     // ---------------- merge the TG warps' states of this piece and write it out
     {
-      float sc = p.scale_log2 * __ldg(p.gk + h);
-      sc = fmaxf(fabsf(sc), 1e-30f);
-      float* ob = obuf + (size_t)w * RP * Sm::OROW;
-#pragma unroll
-      for (int q = 0; q < QT; ++q) {
-#pragma unroll
-        for (int of = 4; of < 32; of <<= 1) {
-          l0[q] += __shfl_xor_sync(0xffffffffu, l0[q], of);
-          l1[q] += __shfl_xor_sync(0xffffffffu, l1[q], of);
-        }
-        const int ra = 8 * q + 2 * c;              // this lane's rows of the tile: ra, ra + 1
-        if (g == 0) {
-          mbuf[w * RP + ra] = m0[q] * sc;          // log2 units from here on
-          mbuf[w * RP + ra + 1] = m1[q] * sc;
-          lbuf[w * RP + ra] = l0[q];
-          lbuf[w * RP + ra + 1] = l1[q];
-        }
-#pragma unroll
-        for (int hf = 0; hf < Gm::NH; ++hf)
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const int ch = 16 * (g + 8 * hf) + 2 * jj;
-            const float* a = o[q][8 * hf + jj];
-            *reinterpret_cast<float2*>(ob + ra * Sm::OROW + ch) = make_float2(a[0], a[2]);
-            *reinterpret_cast<float2*>(ob + (ra + 1) * Sm::OROW + ch) = make_float2(a[1], a[3]);
-          }
-      }
-      __syncthreads();
+      const float sc = fmaxf(fabsf(sc_signed), 1e-30f);
+      constexpr int RM = RP / Sm::MP;                // rows of one merge pass
+      float* ob = obuf + (size_t)w * RM * Sm::OROW;
       const float gvh = __ldg(p.gv + h);
       const int slot_id = part * 2 + (piece_idx == 0 ? 0 : 1);
-      // a thread stays on one query row (4 rows x 32 threads, or 8 x 16), so the warps' weights are worked out once
-      const int tpr = R <= RP / 2 ? NTHREADS / (RP / 2) : NTHREADS / RP;   // threads per row
-      const int row = tid / tpr;
-      if (row < R) {
-        float mx = -3.0e38f;
 #pragma unroll
-        for (int ww = 0; ww < TG; ++ww) mx = fmaxf(mx, mbuf[ww * RP + row]);
-        float den = 0.0f, wgt[TG];
+      for (int mp = 0; mp < Sm::MP; ++mp) {
+        if (Sm::QSM) __syncthreads();                // the query fragments (the rows of the pass before) have been read
 #pragma unroll
-        for (int ww = 0; ww < TG; ++ww) {
-          wgt[ww] = fast_exp2(mbuf[ww * RP + row] - mx);
-          den += lbuf[ww * RP + row] * wgt[ww];
+        for (int q = mp * QT / Sm::MP; q < (mp + 1) * QT / Sm::MP; ++q) {
+#pragma unroll
+          for (int of = 4; of < 32; of <<= 1) {
+            l0[q] += __shfl_xor_sync(0xffffffffu, l0[q], of);
+            l1[q] += __shfl_xor_sync(0xffffffffu, l1[q], of);
+          }
+          const int ra = 8 * q + 2 * c;              // this lane's rows of the tile: ra, ra + 1
+          if (g == 0) {
+            mbuf[w * RP + ra] = m0[q] * sc;          // log2 units from here on
+            mbuf[w * RP + ra + 1] = m1[q] * sc;
+            lbuf[w * RP + ra] = l0[q];
+            lbuf[w * RP + ra + 1] = l1[q];
+          }
+          const int rm = ra - mp * RM;               // .. and of the pass
+#pragma unroll
+          for (int hf = 0; hf < Gm::NH; ++hf)
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              const int ch = 16 * (g + 8 * hf) + 2 * jj;
+              const float* a = o[q][8 * hf + jj];
+              *reinterpret_cast<float2*>(ob + rm * Sm::OROW + ch) = make_float2(a[0], a[2]);
+              *reinterpret_cast<float2*>(ob + (rm + 1) * Sm::OROW + ch) = make_float2(a[1], a[3]);
+            }
         }
-        const float inv = den > 0.0f ? gvh / den : 0.0f;
-        const float* orow = obuf + (size_t)row * Sm::OROW;
-        float* dst_p = nullptr;
-        __nv_bfloat16* dst_o = nullptr;
-        if (complete) {
-          const int t = (p.row0 + row) / G, gq = p.row0 + row - t * G;
-          dst_o = p.out + ((long long)(q0 + t) * (KVH * G) + h * G + gq) * D;
-        } else {
-          dst_p = opart_ws + ((size_t)slot_id * RP + row) * D;
-          if (tid == row * tpr) lse_ws[slot_id * RP + row] = den > 0.0f ? log2f(den) + mx : -__int_as_float(0x7f800000);
-        }
-        for (int ch = (tid - row * tpr) * 2; ch < D; ch += 2 * tpr) {
-          float n0 = 0.0f, n1 = 0.0f;
+        __syncthreads();
+        // a thread stays on one query row (4 rows x 32 threads, or 8 x 16), so the warps' weights are worked out once
+        const int R_here = R - mp * RM;
+        const int tpr = R_here <= RM / 2 ? NTHREADS / (RM / 2) : NTHREADS / RM;   // threads per row
+        const int rl = tid / tpr, row = mp * RM + rl;
+        if (rl < R_here && rl < RM) {
+          float mx = -3.0e38f;
+#pragma unroll
+          for (int ww = 0; ww < TG; ++ww) mx = fmaxf(mx, mbuf[ww * RP + row]);
+          float den = 0.0f, wgt[TG];
 #pragma unroll
           for (int ww = 0; ww < TG; ++ww) {
-            const float2 v = *reinterpret_cast<const float2*>(orow + (size_t)ww * RP * Sm::OROW + ch);
-            n0 += v.x * wgt[ww];
-            n1 += v.y * wgt[ww];
+            wgt[ww] = fast_exp2(mbuf[ww * RP + row] - mx);
+            den += lbuf[ww * RP + row] * wgt[ww];
           }
-          if (complete)
-            *reinterpret_cast<__nv_bfloat162*>(dst_o + ch) = __floats2bfloat162_rn(n0 * inv * p.v_scale, n1 * inv * p.v_scale);
-          else
-            *reinterpret_cast<float2*>(dst_p + ch) = make_float2(n0 * inv, n1 * inv);
+          const float inv = den > 0.0f ? gvh / den : 0.0f;
+          const float* orow = obuf + (size_t)rl * Sm::OROW;
+          float* dst_p = nullptr;
+          __nv_bfloat16* dst_o = nullptr;
+          if (complete) {
+            const int t = (p.row0 + row) / G, gq = p.row0 + row - t * G;
+            dst_o = p.out + ((long long)(q0 + t) * (KVH * G) + h * G + gq) * D;
+          } else {
+            dst_p = opart_ws + ((size_t)slot_id * RP + row) * D;
+            if (tid == rl * tpr) lse_ws[slot_id * RP + row] = den > 0.0f ? log2f(den) + mx : -__int_as_float(0x7f800000);
+          }
+          for (int ch = (tid - rl * tpr) * 2; ch < D; ch += 2 * tpr) {
+            float n0 = 0.0f, n1 = 0.0f;
+#pragma unroll
+            for (int ww = 0; ww < TG; ++ww) {
+              const float2 v = *reinterpret_cast<const float2*>(orow + (size_t)ww * RM * Sm::OROW + ch);
+              n0 += v.x * wgt[ww];
+              n1 += v.y * wgt[ww];
+            }
+            if (complete)
+              *reinterpret_cast<__nv_bfloat162*>(dst_o + ch) = __floats2bfloat162_rn(n0 * inv * p.v_scale, n1 * inv * p.v_scale);
+            else
+              *reinterpret_cast<float2*>(dst_p + ch) = make_float2(n0 * inv, n1 * inv);
+          }
         }
       }
       if (draw_now) __threadfence();                 // this thread's part of the partial, visible device-wide
@@ -904,7 +942,7 @@ int record_cuda(cudaError_t e);
 struct DeviceInfo {
   int sms = 0;
   int ctas_per_sm[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};    // [D == 256][LAYOUT]
-  int ctas_two_tiles = 0;                            // decode_kernel<128, 0, 2>: sixteen query rows per pass
+  int ctas_two_tiles[2] = {0, 0};                    // [D == 256] decode_kernel<D, 0, 2>: sixteen query rows per pass
   std::atomic<bool> ready{false};                    // set (release) after the fields above, under g_setup_mutex
 };
 static DeviceInfo g_dev[64];
@@ -937,7 +975,8 @@ static int device_info(DeviceInfo** out) {
       if ((e = setup_variant<256, 2>(di.ctas_per_sm[1][2])) != cudaSuccess) return record_cuda(e);
       if ((e = setup_variant<128, 3>(di.ctas_per_sm[0][3])) != cudaSuccess) return record_cuda(e);
       if ((e = setup_variant<256, 3>(di.ctas_per_sm[1][3])) != cudaSuccess) return record_cuda(e);
-      if ((e = setup_variant<128, 0, 2>(di.ctas_two_tiles)) != cudaSuccess) return record_cuda(e);
+      if ((e = setup_variant<128, 0, 2>(di.ctas_two_tiles[0])) != cudaSuccess) return record_cuda(e);
+      if ((e = setup_variant<256, 0, 2>(di.ctas_two_tiles[1])) != cudaSuccess) return record_cuda(e);
       di.ready.store(true, std::memory_order_release);
     }
   }
@@ -960,8 +999,8 @@ extern "C" size_t hkv_decode_workspace_bytes(int B, int KVH, int G, int D, int q
   DeviceInfo* di;
   if (device_info(&di) != HKV_OK) return 0;
   size_t need = WorkspaceLayout(max_parts(*di, D), RPAD, D).total;
-  if (D == 128 && G * qlmax > RPAD)                 // head-major pages may take the two-tile kernel (16 rows per pass)
-    need = std::max(need, WorkspaceLayout(std::min(kMaxParts, di->sms * std::max(1, di->ctas_two_tiles)), 2 * RPAD, D).total);
+  if (G * qlmax > RPAD)                             // head-major pages may take the two-tile kernel (16 rows per pass)
+    need = std::max(need, WorkspaceLayout(std::min(kMaxParts, di->sms * std::max(1, di->ctas_two_tiles[D == 256])), 2 * RPAD, D).total);
   return need;
 }
 
@@ -1020,15 +1059,19 @@ static int decode_impl(const void* q, const void* kd, const void* ksf, const voi
   DeviceInfo* di;
   int rc = device_info(&di);
   if (rc != HKV_OK) return rc;
-  // head_dim 128, head-major slot pages, more than 8 query rows per kv head: the two-tile kernel serves 16 rows per pass
-  const bool two = D == 128 && layout == 0 && G * qlmax > RPAD && di->ctas_two_tiles > 0;
+  // head-major slot pages, more than 8 query rows per kv head: the two-tile kernel serves 16 rows per pass
+  bool two = layout == 0 && G * qlmax > RPAD && di->ctas_two_tiles[D == 256] > 0;
+  auto parts_of = [&](int cps) {
+    long long n = std::min<long long>((long long)di->sms * cps, kMaxParts);
+    if (splits > 0) n = std::min<long long>(n, (long long)B * KVH * splits);
+    return n < 1 ? 1 : n;
+  };
+  // (at head_dim 256 its partials may not fit a workspace that is enough for eight rows per pass, e.g. the built-in one)
+  if (two && D == 256 && workspace_bytes < WorkspaceLayout((int)parts_of(di->ctas_two_tiles[1]), 2 * RPAD, D).total) two = false;
   const int rows_per_pass = two ? 2 * RPAD : RPAD;
-  const int cps = two ? di->ctas_two_tiles : di->ctas_per_sm[D == 256][layout];
+  const int cps = two ? di->ctas_two_tiles[D == 256] : di->ctas_per_sm[D == 256][layout];
   if (cps < 1) return HKV_ERR_UNSUPPORTED;
-  (void)max_parts;
-  long long n_parts = std::min<long long>((long long)di->sms * cps, kMaxParts);
-  if (splits > 0) n_parts = std::min<long long>(n_parts, (long long)B * KVH * splits);
-  if (n_parts < 1) n_parts = 1;
+  const long long n_parts = parts_of(cps);
   if (workspace_bytes < WorkspaceLayout((int)n_parts, rows_per_pass, D).total) return HKV_ERR_WORKSPACE;
   DecodeParams p;
   p.q = (const __nv_bfloat16*)q;
@@ -1049,11 +1092,11 @@ static int decode_impl(const void* q, const void* kd, const void* ksf, const voi
   cudaStream_t st = (cudaStream_t)stream;
   const unsigned grid = (unsigned)n_parts;
   void (*k)(const DecodeParams) =
-      two ? decode_kernel<128, 0, 2> :
+      two ? (D == 128 ? decode_kernel<128, 0, 2> : decode_kernel<256, 0, 2>) :
       D == 128 ? (layout == 0 ? decode_kernel<128, 0> : layout == 1 ? decode_kernel<128, 1> : decode_kernel<128, 3>)
                : (layout == 0 ? decode_kernel<256, 0> : layout == 1 ? decode_kernel<256, 1>
                   : layout == 2 ? decode_kernel<256, 2> : decode_kernel<256, 3>);
-  const size_t smem_bytes = two ? (size_t)Smem<128, 0, 2>::TOTAL : D == 128 ? (size_t)Smem<128, 0>::TOTAL
+  const size_t smem_bytes = two ? (size_t)(D == 128 ? Smem<128, 0, 2>::TOTAL : Smem<256, 0, 2>::TOTAL) : D == 128 ? (size_t)Smem<128, 0>::TOTAL
                                      : layout == 2 ? (size_t)Smem<256, 2>::TOTAL : (size_t)Smem<256, 0>::TOTAL;
   static_assert(Smem<128, 0>::TOTAL == Smem<128, 1>::TOTAL && Smem<256, 0>::TOTAL == Smem<256, 1>::TOTAL &&
                 Smem<128, 0>::TOTAL == Smem<128, 3>::TOTAL && Smem<256, 0>::TOTAL == Smem<256, 3>::TOTAL,

@@ -377,3 +377,24 @@ def test_pieces_in_which_some_rows_see_no_key(D):
     assert_close(out, np.nan_to_num(ref2, nan=0.0))
     o2, _ = gpu_decode(c, ws=ws, qlmax=8)
     assert torch.equal(out, o2)
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("KVH,G,ql", [(2, 8, 2), (3, 6, 2), (1, 9, 1), (1, 16, 1), (2, 5, 3), (1, 8, 4), (1, 64, 1)])
+def test_sixteen_rows_per_pass(KVH, G, ql, D):
+    """head-major pages and more than eight query rows per kv head: the two-tile kernel at contexts around its 16- and
+    32-token blocks, against the oracle; at head_dim 256 a workspace that only holds eight rows' partials (what a caller
+    without extra rows allocates) takes eight rows per pass and gives the same within the tolerance"""
+    lens = [max(ql, n) for n in (1, 15, 16, 17, 31, 32, 33, 700, 2050)]
+    c = build_decode_case(2600 + G, lens, KVH, G, D, 16, ql_list=[ql] * len(lens))
+    ref = oracle_decode(c)
+    out, ws = gpu_decode(c, qlmax=ql)
+    assert K.workspace_status(ws) == 0
+    assert_close(out, ref, "sixteen rows per pass")
+    again, _ = gpu_decode(c, qlmax=ql, ws=ws)
+    assert torch.equal(out, again)
+    if D == 256:
+        small = K.alloc_workspace(len(lens), KVH, 8, D, 1)
+        assert small.numel() < K.workspace_bytes(len(lens), KVH, G, D, ql)
+        eight, _ = gpu_decode(c, qlmax=ql, ws=small)
+        assert_close(eight, ref, "eight rows per pass")
