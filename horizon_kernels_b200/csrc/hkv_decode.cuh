@@ -1,5 +1,4 @@
-// Declarations shared by the two decode kernels (hkv_decode.cu: warp-level mma.sync path for every cache layout;
-// hkv_decode_umma.cu: tcgen05 path for head-major slot pages): launch parameters, the per-request view of the unit
+// Declarations of the decode kernel (hkv_decode.cu): launch parameters, the per-request view of the unit
 // stream, and the log-sum-exp merge of a split sequence.
 #pragma once
 
