@@ -342,7 +342,7 @@ def _build_classes():
             memory held. Causal window of the reference: query token t of ql sees keys j < L - ql + t + 1. The score
             product takes bf16 queries as they are (the reference's default converts them to fp16, backend.py:229; code *
             scale is exact in both) and other types converted to fp16 (HORIZON_KVFP4_PF16=1) or bf16; the value product
-            takes fp16 operands (the dequantised values are exact in it and the probabilities lie in [0, 2^14]); both
+            takes fp16 operands (the dequantised values are exact in it and the probabilities lie in [0, 1]); both
             accumulate in fp32. The global scales are folded into the softmax scale and the output like the reference's
             sm / vs."""
             rows = [(row, q0, q1, L) for row, q0, q1, L in m.prefill_rows if q1 > q0 and L > 0]

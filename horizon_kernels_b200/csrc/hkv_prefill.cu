@@ -28,7 +28,6 @@ constexpr int kPfCtas = 160;           // CTAs per launch
 constexpr int kKeys = 128;             // keys per tile
 constexpr int kPieceCost = 3;          // cost of starting and ending a piece, in key tiles (of about 1 us)
 constexpr int kMinPiece = 2;           // no piece of a divided row tile is shorter, in key tiles
-constexpr float kMaxLag = 14.0f;        // log2 by which a score may exceed the running maximum: probabilities stay inside f16
 constexpr int kStageBytes = 32768;
 constexpr int kStages = 5;
 constexpr uint32_t kQBytes = 65536;    // query operands of 128 rows: two buffers at head_dim 128, one at 256
@@ -307,19 +306,9 @@ __device__ __forceinline__ void tm_ld32(uint32_t* x, uint32_t addr) {
       : HKV_R32(x)
       : "r"(addr));
 }
-__device__ __forceinline__ void tm_ld16(uint32_t* x, uint32_t addr) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
-                 "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-               : "r"(addr));
-}
 __device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // keeps the uses of loaded registers behind the wait (an empty statement that passes them through)
 __device__ __forceinline__ void tm_ready(uint32_t* x) { asm volatile("" : HKV_RW32(x)); }
-__device__ __forceinline__ void tm_ready16(uint32_t* x) {
-  asm volatile("" : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(x[8]),
-                    "+r"(x[9]), "+r"(x[10]), "+r"(x[11]), "+r"(x[12]), "+r"(x[13]), "+r"(x[14]), "+r"(x[15]));
-}
 __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t* x) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::HKV_I16(x),
@@ -415,9 +404,13 @@ __device__ __forceinline__ void store_out(const PrefillParams& p, long long elem
 // of the time (3590 clocks for both against 2048; here 1450 a tile) and 9000 clocks between pieces (here about 3000; short
 // prompts gain most, a step of four prompts with 48 decode requests went from 128 to 117 us); 64-key steps with two buffers
 // each paid twice for the score product, which reads its 128 query rows from shared memory whatever the number of keys.
-// The 16-bit probabilities go over the scores they came from. The running maximum moves only when a score exceeds it by
-// 2^14 (the probabilities then stay below 2^14, inside f16), so the output is hardly ever rescaled; a thread tells the next
-// tile's thread of its row the maximum as soon as it knows it.
+// The 16-bit probabilities go over the scores they came from. A thread tells the next tile's thread of its row the running
+// maximum as soon as it knows it, and rescales the output, where the maximum has moved, after its probabilities are written:
+// the wait for the value product before it then passes behind the exponentials. The maximum is the exact one: the largest
+// probability is 1 and loses nothing to the rounding to f16. One that lags by up to 2^14 hardly ever rescales, but its
+// largest probability is any number: the error against 64 bits (before the output's own rounding) was 1.9e-4 where this has
+// 6.5e-5 (a prompt of 6144 tokens, head_dim 128: 324 us either way; 518 us with the rescaling before the exponentials) and
+// 2.0e-4 where this has 8.3e-5 (2048 tokens over 30000, head_dim 256: 735 us there, 770 here).
 // A walk over the CTA's key tiles, piece by piece. A step to the next row tile of a request costs a few instructions: every
 // role takes it at every piece, two of them in a single thread.
 struct Tiles {
@@ -831,31 +824,15 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
         if (g > 0) ok = all_wait(word_before, (g - 1) / SETS);
         if (!ok) break;
         const float m_old = m, m_in = head ? -INFINITY : *top_now;
-        const bool move = top > m_in + kMaxLag;
+        const bool move = top > m_in;
         m = move ? (top == INFINITY ? 0.0f : top) : m_in;
         if (move || head) *top_now = m;
         mbar_arrive_u32(my_word);
         if (__any_sync(0xffffffffu, m != m_old)) {
           const float al = m == m_old ? 1.0f : fast_exp2(m_old - m);
           l2 = mul2(l2, pack2(al, al));
-          if (!head && __any_sync(0xffffffffu, move)) {
-            // the output of the tiles before this one, all of whose value products must have been added first
-            ok = all_wait(o_done0 + 8 * before, (g - 1) / SETS);
-            if (!ok) break;
-            tc_fence_after();
-            const float al_o = move ? fast_exp2(m_in - m) : 1.0f;
-#pragma unroll 1
-            for (int i = 0; i < D; i += 16) {
-              uint32_t o[16];
-              tm_ld16(o, lane_base + S::OCOL + i);
-              tm_wait_ld();
-              tm_ready16(o);
-#pragma unroll
-              for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * al_o);
-              tm_st16(lane_base + S::OCOL + i, o);
-            }
-          }
         }
+        const float al_o = move && !head ? fast_exp2(m_in - m) : 1.0f;
         const float mu = m == -INFINITY ? 0.0f : -m;
         const unsigned long long c2 = pack2(p.c, p.c), m2 = pack2(mu, mu);
         // from the last 32 scores (still in registers) to the first, so that the probabilities of a part, 16 columns, go over
@@ -875,6 +852,37 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
           tm_st16(s_addr + 64 + 16 * c, ph16);
           if (c == 0) break;
           load(c - 1);
+        }
+        if (__any_sync(0xffffffffu, al_o != 1.0f)) {
+          // the output of the tiles before this one, all of whose value products must have been added first; 64 columns at a
+          // time and in packed pairs (32 at a time, one by one: 787 us where this takes 770, head_dim 256)
+          ok = all_wait(o_done0 + 8 * before, (g - 1) / SETS);
+          if (!ok) {
+            tc_wait_st();
+            break;
+          }
+          tc_fence_after();
+          const unsigned long long al2 = pack2(al_o, al_o);
+#pragma unroll 1
+          for (int i = 0; i < D; i += 64) {
+            uint32_t o[2][32];
+            tm_ld32(o[0], lane_base + S::OCOL + i);
+            tm_ld32(o[1], lane_base + S::OCOL + i + 32);
+            tm_wait_ld();
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              tm_ready(o[u]);
+#pragma unroll
+              for (int k = 0; k < 32; k += 2) {
+                float a, b;
+                unpack2(mul2(pack2(__uint_as_float(o[u][k]), __uint_as_float(o[u][k + 1])), al2), a, b);
+                o[u][k] = __float_as_uint(a);
+                o[u][k + 1] = __float_as_uint(b);
+              }
+              tm_st16(lane_base + S::OCOL + i + 32 * u, o[u]);
+              tm_st16(lane_base + S::OCOL + i + 32 * u + 16, o[u] + 16);
+            }
+          }
         }
         tc_wait_st();
         tc_fence_before();

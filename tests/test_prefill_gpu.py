@@ -128,3 +128,92 @@ def test_graph_capture_and_repeat():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, eager)
+
+
+def filled(KVH, D, L, k, v, gk, PS=16, n_req=1):
+    """head-major cache of n_req requests of L tokens with the given keys and values, (flat, strides), block tables"""
+    dev = torch.device("cuda")
+    per = (L + PS - 1) // PS
+    cache = Lt.alloc_cache(per * n_req + 2, PS, KVH, D, device=dev, fill=0x7F)
+    flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
+    bt = torch.randperm(per * n_req, device=dev).to(torch.int32).view(n_req, per)
+    pos = torch.arange(L, device=dev)
+    slots = (bt[:, pos // PS].long() * PS + pos % PS).reshape(-1)
+    one = torch.ones(KVH, device=dev)
+    K.write(k.to(torch.bfloat16), v.to(torch.bfloat16), flat, strides, PS, slots, gk * one, one)
+    return flat, strides, bt
+
+
+def attend64(q, flat, strides, PS, bt, rows, KVH, sm, f16_probabilities=False):
+    """per (token, head) in 64 bits: the output, sum_j w_j |v_j|, and the largest score (log2) of every 128 keys; optionally
+    with the probabilities rounded to f16 under the row's exact maximum before the value product"""
+    NT, HQ, D = q.shape
+    G = HQ // KVH
+    out, absv = (torch.zeros(NT, HQ, D, dtype=torch.float64, device=q.device) for _ in range(2))
+    tops = {}
+    for b, q0, q1, L in rows:
+        kk, vv = (torch.empty(L, KVH, D, dtype=torch.float16, device=q.device) for _ in range(2))
+        K.dequant_tokens(flat, strides, PS, bt[b].contiguous(), 0, L, kk, vv)
+        ql = q1 - q0
+        hidden = torch.arange(L, device=q.device)[None] >= torch.arange(L - ql + 1, L + 1, device=q.device).repeat_interleave(G)[:, None]
+        for h in range(KVH):
+            s = q[q0:q1, h * G:(h + 1) * G].reshape(ql * G, D).double() @ kk[:, h].double().T * sm
+            s.masked_fill_(hidden, -float("inf"))
+            p = torch.exp(s - s.amax(dim=1, keepdim=True))
+            pn = p.half().double() if f16_probabilities else p
+            den = p.sum(dim=1, keepdim=True)
+            out[q0:q1, h * G:(h + 1) * G] = (pn @ vv[:, h].double() / den).view(ql, G, D)
+            absv[q0:q1, h * G:(h + 1) * G] = (p @ vv[:, h].double().abs() / den).view(ql, G, D)
+            pad = torch.nn.functional.pad(s, (0, -L % 128), value=-float("inf"))
+            tops[b, h] = pad.view(ql * G, -1, 128).amax(dim=2) * 1.4426950408889634
+    return out, absv, tops
+
+
+@pytest.mark.parametrize("KVH,G,D,ql,L,amp", [(2, 4, 128, 700, 3000, 1.0), (2, 8, 256, 256, 5000, 1.0), (1, 4, 128, 5, 9000, 1.0),
+                                              (2, 4, 128, 512, 4000, 0.3), (2, 4, 256, 300, 4000, 0.1)])
+def test_error_is_that_of_probabilities_under_the_exact_maximum(KVH, G, D, ql, L, amp):
+    """fp32 output against 64 bits: what the products lose is the rounding of the probabilities to f16. Where few keys have most
+    of the weight it is small if the largest probability is exactly 1, as under the row's exact maximum, and two to three times
+    that under a maximum that lags behind. The bound is the error of 64-bit attention with probabilities rounded to f16 under the
+    exact maximum, plus a tenth (the running maximum rounds the earlier keys on another grid)"""
+    g = torch.Generator(device="cuda").manual_seed(D + ql)
+    k, v = torch.randn(2, L, KVH, D, generator=g, device="cuda")
+    k[:, :, [3, D // 4 + 3, D // 2 + 3, 3 * D // 4 + 3]] *= 20.0 * amp
+    flat, strides, bt = filled(KVH, D, L, k, v, 0.04)
+    q = torch.randn(ql, KVH * G, D, generator=g, device="cuda").to(torch.bfloat16)
+    rows, sm = [(0, 0, ql, L)], D ** -0.5 * 0.04
+    out = torch.zeros(ql, KVH * G, D, device="cuda")
+    K.prefill(q, flat, strides, 16, bt, rows, sm, 1.0, KVH, out)
+    want, _, _ = attend64(q, flat, strides, 16, bt, rows, KVH, sm)
+    f16, _, _ = attend64(q, flat, strides, 16, bt, rows, KVH, sm, f16_probabilities=True)
+    err, bound = (out.double() - want).norm() / want.norm(), (f16 - want).norm() / want.norm()
+    assert err <= 1.1 * bound, (float(err), float(bound))
+
+
+@pytest.mark.parametrize("KVH,G,D,ql,L,chunk", [(2, 4, 128, 1100, 2200, 65536), (2, 4, 128, 1100, 2200, 512), (1, 4, 128, 9, 1700, 65536),
+                                                (2, 8, 256, 560, 1700, 65536), (2, 8, 256, 560, 1700, 512), (1, 8, 256, 9, 1700, 65536),
+                                                (1, 8, 256, 9, 1700, 900)])
+def test_maxima_that_rise_in_every_tile(KVH, G, D, ql, L, chunk):
+    """keys that grow along the context: for every other query head each tile's largest score exceeds all before it by more than
+    14 (log2), for the rest it falls, so that in every tile some rows of a warp rescale the output and others do not; row tiles
+    whole (6 tiles and more), divided among CTAs, and chunk by chunk. Every element against 64 bits"""
+    g = torch.Generator(device="cuda").manual_seed(D + ql + chunk)
+    u = torch.nn.functional.normalize(torch.randn(KVH, D, generator=g, device="cuda"), dim=1)
+    grow = (torch.arange(L, device="cuda") // 128 + 1).float()[:, None, None]
+    k = u * grow * 3.0 + 0.02 * torch.randn(L, KVH, D, generator=g, device="cuda")
+    v = torch.randn(L, KVH, D, generator=g, device="cuda")
+    flat, strides, bt = filled(KVH, D, L, k, v, float(k.abs().max()) / 2688)
+    sign = 1.0 - 2.0 * (torch.arange(KVH * G, device="cuda") % 2)
+    q = (u.repeat_interleave(G, dim=0) * sign[:, None] + 0.01 * torch.randn(ql, KVH * G, D, generator=g, device="cuda")).to(torch.bfloat16)
+    rows, sm = [(0, 0, ql, L)], 6.0 * float(k.abs().max()) / 2688
+    out = torch.zeros(ql, KVH * G, D, device="cuda")
+    K.prefill(q, flat, strides, 16, bt, rows, sm, 1.0, KVH, out, chunk=chunk)
+    want, absv, tops = attend64(q, flat, strides, 16, bt, rows, KVH, sm)
+    for t in tops.values():                              # [token x head][tile]; the first eight tiles are whole for every row
+        t = t.view(ql, G, -1)[:, :, :8]
+        assert (t[:, 0::2].diff(dim=2) > 14).all() and (t[:, 1::2].diff(dim=2) < 0).all()
+    # a weight is off by 2^-11 from f16 and by less than 2^-12 from its exponent (scores below 500 (log2), fp32 sums of products);
+    # probabilities below f16's normal range by 2^-25 of the largest
+    bound = absv * (2.0 ** -11 + 2.0 ** -12) + L * 2.0 ** -25 * float(v.abs().max()) * 2
+    bad = ((out.double() - want).abs() > bound).sum()
+    assert bad == 0, int(bad)
