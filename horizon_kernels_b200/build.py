@@ -36,7 +36,7 @@ def _run(cmd, verbose=False):
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OUT_DIR, exist_ok=True)
     src = _newest_source()
-    if force or not os.path.exists(HOST) or os.path.getmtime(HOST) < src:
+    if force or not os.path.exists(HOST) or os.path.getmtime(HOST) < src or not _host_loads():
         build_host()
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= src:
         return LIB
@@ -46,6 +46,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def _host_loads() -> bool:
+    """whether the built host module is one for the installed torch"""
+    from . import _lib
+    try:
+        _lib.load_host(HOST)
+        return True
+    except (ImportError, OSError, AttributeError):
+        return False
+
+
 def build_host() -> str:
     import sysconfig
 
@@ -53,7 +63,8 @@ def build_host() -> str:
     t = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
     _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{t}/include",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          f'-DHKV_TORCH_VERSION="{torch.__version__}"', f"-I{t}/include",
           f"-I{t}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
           os.path.join(CSRC, "hkv_host.cpp"), "-o", HOST, f"-L{t}/lib", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
           "-ltorch_python"])

@@ -270,4 +270,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "hkv_host", nullptr, -1, methods, n
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_hkv_host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit_hkv_host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch_version", HKV_TORCH_VERSION) != 0) {   // the torch it is compiled against
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}
