@@ -1150,7 +1150,7 @@ extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void*
   }
   const float c = qk_scale * 1.4426950408889634f;
   p.c = fmaxf(fabsf(c), 1e-37f);                          // (zero: masked scores would become 0 * -inf)
-  p.vs = out_scale;
+  p.vs = c != c ? c : out_scale;                          // (fmaxf drops a NaN: the output takes it instead)
   p.out = out;
   p.out_f32 = out_f32;
   p.k_bf16 = !q_f16;                                      // (the cached values are exact in both types)

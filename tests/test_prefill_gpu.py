@@ -217,3 +217,24 @@ def test_maxima_that_rise_in_every_tile(KVH, G, D, ql, L, chunk):
     bound = absv * (2.0 ** -11 + 2.0 ** -12) + L * 2.0 ** -25 * float(v.abs().max()) * 2
     bad = ((out.double() - want).abs() > bound).sum()
     assert bad == 0, int(bad)
+
+
+@pytest.mark.parametrize("ql,L,chunk", [(300, 900, 65536), (6, 3000, 65536), (200, 1000, 256)])
+@pytest.mark.parametrize("D", [128, 256])
+def test_non_finite_queries_and_scales(D, ql, L, chunk):
+    """row tiles whole, divided and chunk by chunk: a query row with a NaN or an infinity gives NaN, as softmax over its scores
+    does, and changes no other row; a NaN scale gives NaN"""
+    KVH, G = 1, 4
+    g = torch.Generator(device="cuda").manual_seed(D + ql)
+    k, v = torch.randn(2, L, KVH, D, generator=g, device="cuda")
+    flat, strides, bt = filled(KVH, D, L, k, v, 0.01)
+    q = torch.randn(ql, KVH * G, D, generator=g, device="cuda").to(torch.bfloat16)
+    call = lambda q, a, b: K.prefill(q, flat, strides, 16, bt, [(0, 0, ql, L)], a, b, KVH, torch.zeros_like(q), chunk=chunk)  # noqa: E731
+    want, bad = call(q, D ** -0.5, 1.0), q.clone()
+    bad[0, 1, 5], bad[3, 0, 0], bad[ql - 1, 3, D - 1] = float("nan"), float("inf"), float("-inf")
+    hit = torch.zeros(ql, KVH * G, dtype=torch.bool, device="cuda")
+    hit[0, 1] = hit[3, 0] = hit[ql - 1, 3] = True
+    got = call(bad, D ** -0.5, 1.0)
+    assert got[hit].isnan().all() and torch.equal(got[~hit], want[~hit]) and torch.isfinite(want.float()).all()
+    for a, b in ((float("nan"), 1.0), (1.0, float("nan"))):
+        assert call(q, a, b).isnan().all(), (a, b)
