@@ -14,7 +14,7 @@ EXPORTS = ("hkv_version", "hkv_error_string", "hkv_last_cuda_error", "hkv_write"
            "hkv_set_option", "hkv_dequant", "hkv_write_rot",
            "hkv_decode_rot", "hkv_write_k8", "hkv_decode_k8", "hkv_dequant_k8",
            "hkv_prefill", "hkv_prefill_scratch_bytes",
-           "hkv_selftest_wait_timeout", "hkv_selftest_codec", "hkv_probe_issue_rates")
+           "hkv_selftest_wait_timeout", "hkv_selftest_prefill_timeout", "hkv_selftest_codec", "hkv_probe_issue_rates")
 
 _lib = None
 _host = None
@@ -75,9 +75,10 @@ def load():
                                      i32, vp]
         L.hkv_prefill_scratch_bytes.restype = C.c_size_t
         L.hkv_prefill_scratch_bytes.argtypes = [C.POINTER(i32), i32, i32, i32, i32, i32, i64, i32]
-        L.hkv_prefill.restype = i32
+        L.hkv_prefill.restype = L.hkv_selftest_prefill_timeout.restype = i32
         L.hkv_prefill.argtypes = [vp, i32, vp, vp, vp, vp, C.POINTER(i64), i32, vp, i32, i32, C.POINTER(i32), i32, i32, i32,
                                   i32, i32, f32, f32, vp, i32, i64, vp, C.c_size_t, vp, i32, vp, vp]
+        L.hkv_selftest_prefill_timeout.argtypes = L.hkv_prefill.argtypes
         L.hkv_selftest_wait_timeout.restype = i32
         L.hkv_selftest_wait_timeout.argtypes = [vp, i64, vp]
         L.hkv_selftest_codec.restype = i32

@@ -1206,6 +1206,23 @@ constexpr size_t kNoAllocScratchBytes = 5u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 // device address of the array per device ordinal; the symbol's name above is only a host-side handle
 static std::atomic<void*> g_noalloc_ptr[64] = {};
+
+// that address for the current device
+int noalloc_workspace(void** out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return record_cuda(e);
+  if (dev < 0 || dev >= 64) return HKV_ERR_RANGE;
+  void* ws = g_noalloc_ptr[dev].load(std::memory_order_acquire);
+  if (ws == nullptr) {                              // set-up, once per device, with that device current
+    e = cudaGetSymbolAddress(&ws, g_noalloc_scratch);
+    if (e != cudaSuccess) return record_cuda(e);
+    if (ws == nullptr) return HKV_ERR_CUDA;
+    g_noalloc_ptr[dev].store(ws, std::memory_order_release);   // (two threads racing here store the same address)
+  }
+  *out = ws;
+  return HKV_OK;
+}
 }  // namespace hkv
 
 extern "C" int hkv_decode_noalloc(const void* q, const void* kd, const void* ksf, const void* vd, const void* vsf,
@@ -1219,19 +1236,11 @@ extern "C" int hkv_decode_noalloc(const void* q, const void* kd, const void* ksf
   if (D != 128 && D != 256) return HKV_ERR_UNSUPPORTED;
   if (KVH < 1 || G < 1 || qlmax < 1 || G * qlmax > kMaxRows) return HKV_ERR_UNSUPPORTED;
   if (splits > 64) return HKV_ERR_SPLITS;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return record_cuda(e);
-  if (dev < 0 || dev >= 64) return HKV_ERR_RANGE;
-  void* ws = g_noalloc_ptr[dev].load(std::memory_order_acquire);
-  if (ws == nullptr) {                              // set-up, once per device, with that device current
-    e = cudaGetSymbolAddress(&ws, g_noalloc_scratch);
-    if (e != cudaSuccess) return record_cuda(e);
-    if (ws == nullptr) return HKV_ERR_CUDA;
-    g_noalloc_ptr[dev].store(ws, std::memory_order_release);   // (two threads racing here store the same address)
-  }
+  void* ws;
+  int rc0 = noalloc_workspace(&ws);
+  if (rc0 != HKV_OK) return rc0;
   DeviceInfo* di;
-  const int rc0 = device_info(&di);
+  rc0 = device_info(&di);
   if (rc0 != HKV_OK) return rc0;
   // the scratch a call needs grows with the number of stream partitions, which is bounded by the device's resident
   // CTAs and by B * KVH * splits
@@ -1253,7 +1262,7 @@ extern "C" int hkv_decode_noalloc_status(int* status, void* stream) {
   if (e != cudaSuccess) return record_cuda(e);
   if (dev < 0 || dev >= 64) return HKV_ERR_RANGE;
   void* ws = g_noalloc_ptr[dev].load(std::memory_order_acquire);
-  if (ws == nullptr) {                              // no hkv_decode_noalloc call on this device yet: nothing to report
+  if (ws == nullptr) {                              // neither hkv_decode_noalloc nor hkv_prefill without a workspace on this device yet: nothing to report
     *status = HKV_OK;
     return HKV_OK;
   }

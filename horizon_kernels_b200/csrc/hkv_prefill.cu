@@ -22,6 +22,7 @@
 namespace hkv {
 
 int record_cuda(cudaError_t e);
+int noalloc_workspace(void** ws);
 
 constexpr int kPfReqs = 32;            // requests per launch (the tables below are kernel arguments, at most 4 KB)
 constexpr int kPfCtas = 160;           // CTAs per launch
@@ -63,7 +64,7 @@ struct PrefillParams {
   float* part_ml;                      // [CTA][2][2][128]: running maximum (log2 domain), sum
   float* state_o;                      // chunked contexts: [token][head][D], then the same tables per row
   float* state_ml;
-  int* status;
+  int* status;                         // of the workspace, or of the built-in one
   float c, vs;                         // score scale x log2(e) (> 0), output scale
   int out_f32, k_bf16;
   int KVH, G, tok;                     // tok: query tokens per row tile (128 / G)
@@ -357,20 +358,22 @@ constexpr int kPfSmem = (int)kQBytes + kStages * kStageBytes + kAux + (int)sizeo
 static_assert(kPfSmem <= 232448, "shared memory");
 
 // bounded wait: gives up when it runs out or when another role of the CTA has given up
+template <long long LIMIT>
 __device__ __forceinline__ bool pf_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort) {
   const long long t0 = clock64();
   while (!mbar_try_wait_u32(bar, parity)) {
     if (*abort) return false;
-    if (clock64() - t0 > kWaitCycles) {
+    if (clock64() - t0 > LIMIT) {
       *abort = 1;
       return false;
     }
   }
   return true;
 }
+template <long long LIMIT>
 __device__ __forceinline__ bool pf_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
   if (mbar_try_wait_u32(bar, parity)) return true;
-  return pf_wait_slow(bar, parity, abort);
+  return pf_wait_slow<LIMIT>(bar, parity, abort);
 }
 
 __device__ __forceinline__ void store_out(const PrefillParams& p, long long elem, const float* v) {   // 8 values
@@ -469,12 +472,14 @@ struct Tiles {
   }
 };
 
-template <int D>
+// LOSE (the self-test of the give-up path): the copy warp stops after three stages, and waits run out after a millisecond.
+template <int D, bool LOSE>
 __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __grid_constant__ PrefillParams p) {
   using S = PfShape<D>;
   constexpr int SETS = S::SETS, SOFT = S::SOFT, NQ = S::NQ;
   constexpr uint32_t IMAGE = kKeys * D * 2;
   constexpr int PER = IMAGE / kStageBytes;                // ring stages per operand tile: 1 or 2
+  constexpr long long LIMIT = LOSE ? 1ll << 21 : kWaitCycles;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* ring = smem + kQBytes;
   uint8_t* aux = smem + kQBytes + kStages * kStageBytes;
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
                  q_free0 = smem_u32(&sh.q_free[0]), s_full0 = smem_u32(&sh.s_full[0]), p_full0 = smem_u32(&sh.p_full[0]),
                  o_done0 = smem_u32(&sh.o_done[0]), told0 = smem_u32(&sh.told[0]), ml_full = smem_u32(&sh.ml_full),
                  ml_free = smem_u32(&sh.ml_free), o_free = smem_u32(&sh.o_free);
-  auto all_wait = [&](uint32_t bar, uint32_t phase) { return (bool)__all_sync(0xffffffffu, pf_wait(bar, phase & 1, abort)); };
+  auto all_wait = [&](uint32_t bar, uint32_t phase) { return (bool)__all_sync(0xffffffffu, pf_wait<LIMIT>(bar, phase & 1, abort)); };
 
   if (warp == SOFT + 1) {
     // ------------------------------------------------------------------------------------------------ copy warp
@@ -524,7 +529,8 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
         const int n_t = min(p.kt_hi, (r.L + kKeys - 1) / kKeys) - p.kt_lo;
         const uint8_t* from = p.tiles + ((size_t)r.tile0 * p.KVH + (size_t)x.h * n_t + (x.kt - p.kt_lo)) * 2 * IMAGE + side * IMAGE;
         for (int i = 0; ok && i < PER; ++i) {
-          if (turn > 0) ok = pf_wait(empty0 + 8 * st, (turn - 1) & 1, abort);
+          if (LOSE && fill == 3) ok = false;
+          else if (turn > 0) ok = pf_wait<LIMIT>(empty0 + 8 * st, (turn - 1) & 1, abort);
           if (!ok) return;
           mbar_expect_tx_u32(full0 + 8 * st, kStageBytes);
           bulk_g2s_u32(smem_u32(ring) + st * kStageBytes, from + i * kStageBytes, kStageBytes, full0 + 8 * st);
@@ -538,10 +544,9 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
         if (!k.end) fetch(k, 0);
         if (ok) fetch(v, 1);
       }
-      if (!ok) {                       // nothing of this CTA's may still be on its way when it ends
-        for (uint32_t f = fill > kStages ? fill - kStages : 0; f < fill; ++f)
-          mbar_wait_bounded_u32(full0 + 8 * (f % kStages), (f / kStages) & 1);
-      }
+      // nothing of this CTA's may still be on its way when it ends (another role may give up at any time)
+      for (uint32_t f = fill > kStages ? fill - kStages : 0; f < fill; ++f)
+        mbar_wait_bounded_u32(full0 + 8 * (f % kStages), (f / kStages) & 1);
     }
   } else if (warp == SOFT) {
     // ------------------------------------------------------------------------------------------------- MMA warp
@@ -554,14 +559,14 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
       uint32_t use = 0;                                   // ring stages handed out, in the copy warp's order
       uint32_t sk = 0, sv = 0, tv = 0;                    // score tile (of SETS) of the next score and value product; turn of the latter
       bool ok = *abort == 0;
-      auto stage_wait = [&](uint32_t n) { return pf_wait(full0 + 8 * (n % kStages), (n / kStages) & 1, abort); };
+      auto stage_wait = [&](uint32_t n) { return pf_wait<LIMIT>(full0 + 8 * (n % kStages), (n / kStages) & 1, abort); };
       auto stage_addr = [&](uint32_t n) { return ring_a + (n % kStages) * kStageBytes; };
       auto stages_done = [&](uint32_t n) {
         for (int i = 0; i < PER; ++i) umma_commit(empty0 + 8 * ((n + i) % kStages));
       };
       auto scores = [&](uint32_t n) {                     // of the next key tile, which lies in stage n (and n + 1)
         const uint32_t qb = k.piece % NQ;
-        if (k.first) ok = pf_wait(q_full0 + 8 * qb, (k.piece / NQ) & 1, abort);
+        if (k.first) ok = pf_wait<LIMIT>(q_full0 + 8 * qb, (k.piece / NQ) & 1, abort);
         ok = ok && stage_wait(n) && (PER == 1 || stage_wait(n + 1));
         if (!ok) return;
         tc_fence_after();
@@ -581,7 +586,7 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
       auto values = [&](uint32_t n) {
         // (the accumulator holds the piece before until the end warps have read it)
         ok = stage_wait(n) && (PER == 1 || stage_wait(n + 1)) &&
-             (!v.first || v.piece == 0 || pf_wait(o_free, (v.piece - 1) & 1, abort)) && pf_wait(p_full0 + 8 * sv, tv & 1, abort);
+             (!v.first || v.piece == 0 || pf_wait<LIMIT>(o_free, (v.piece - 1) & 1, abort)) && pf_wait<LIMIT>(p_full0 + 8 * sv, tv & 1, abort);
         if (!ok) return;
         tc_fence_after();
 #pragma unroll
@@ -610,10 +615,9 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
         if (ok && !later) values(use + PER);
         use += 2 * PER;
       }
-      if (!ok) {                       // no product of this CTA's may still be running when its tensor memory is given back
-        umma_commit(smem_u32(&sh.drain));
-        mbar_wait_bounded_u32(smem_u32(&sh.drain), 0);
-      }
+      // no product of this CTA's may still be running when its tensor memory is given back
+      umma_commit(smem_u32(&sh.drain));
+      mbar_wait_bounded_u32(smem_u32(&sh.drain), 0);
     }
   } else if (warp >= SOFT + 4) {
     // ------------------------------------------------------------------------------------------------ end warps
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
       const int ch = row % LPR, tok0 = y.rt * p.tok;
       const uint32_t qs = smem_u32(smem) + (y.piece % NQ) * 32768 + (ch >> 3) * 16384;
       const uint16_t* q = (const uint16_t*)p.q + ((long long)(r.q0 + tok0) * HQ + y.h * p.G) * D + ch * 8;
-      if (y.piece >= NQ && !pf_wait(q_free0 + 8 * (y.piece % NQ), (y.piece / NQ - 1) & 1, abort)) return false;
+      if (y.piece >= NQ && !pf_wait<LIMIT>(q_free0 + 8 * (y.piece % NQ), (y.piece / NQ - 1) & 1, abort)) return false;
 #pragma unroll 4
       for (int rr = row / LPR; rr < 128; rr += RSTEP) {
         const int tk = (int)((uint32_t)rr * inv_g >> 16);
@@ -916,7 +920,7 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
   __syncthreads();
   tc_fence_after();
   if (warp == SOFT) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
-  if (tid == 0 && *abort && p.status != nullptr) atomicExch(p.status, HKV_ERR_DEVICE_WAIT);
+  if (tid == 0 && *abort) atomicExch(p.status, HKV_ERR_DEVICE_WAIT);
 }
 
 // ------------------------------------------------------------------------------------------------------ merge_kernel
@@ -1112,11 +1116,11 @@ extern "C" size_t hkv_prefill_scratch_bytes(const int32_t* rows, int n_rows, int
   return prefill_scratch(rows, n_rows, n_tokens, KVH, G, D, chunk_tiles_of(chunk), rotated).total;
 }
 
-extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
+static int prefill_impl(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
                            const int64_t strides[6], int PS, const int32_t* block_tables, int n_tables, int MP,
                            const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale,
                            const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out,
-                           int out_f32, void* workspace, void* stream) {
+                           int out_f32, void* workspace, void* stream, bool lose) {
   using namespace hkv;
   if (n_rows == 0) return HKV_OK;
   if (n_rows < 0) return HKV_ERR_RANGE;
@@ -1160,7 +1164,11 @@ extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void*
   p.tiles = base + sc.tiles;
   p.part_o = (float*)(base + sc.part_o);
   p.part_ml = (float*)(base + sc.part_ml);
-  p.status = workspace ? &((Header*)workspace)->status : nullptr;
+  if (!workspace) {
+    rc = noalloc_workspace(&workspace);
+    if (rc != HKV_OK) return rc;
+  }
+  p.status = &((Header*)workspace)->status;
   const int n_cta = prefill_ctas();
 
   TileParams t = {};
@@ -1174,7 +1182,8 @@ extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void*
   if (k8) tk = q_f16 ? tile_kernel<256, 0, 1> : tile_kernel<256, 1, 1>;
   else if (D == 128) tk = q_f16 ? tile_kernel<128, 0, 0> : tile_kernel<128, 1, 0>;
   else tk = q_f16 ? tile_kernel<256, 0, 0> : tile_kernel<256, 1, 0>;
-  void (*ak)(const PrefillParams) = D == 128 ? attend_kernel<128> : attend_kernel<256>;
+  void (*ak)(const PrefillParams) = lose ? (D == 128 ? attend_kernel<128, true> : attend_kernel<256, true>)
+                                         : D == 128 ? attend_kernel<128, false> : attend_kernel<256, false>;
   void (*mk)(const PrefillParams) = D == 128 ? merge_kernel<128> : merge_kernel<256>;
   rc = record_cuda(cudaFuncSetAttribute((const void*)ak, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
   if (rc != HKV_OK) return rc;
@@ -1212,4 +1221,23 @@ extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void*
     i += g.n;
   }
   return HKV_OK;
+}
+
+extern "C" int hkv_prefill(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
+                           const int64_t strides[6], int PS, const int32_t* block_tables, int n_tables, int MP,
+                           const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale,
+                           const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out,
+                           int out_f32, void* workspace, void* stream) {
+  return prefill_impl(q, q_f16, kd, ksf, vd, vsf, strides, PS, block_tables, n_tables, MP, rows, n_rows, n_tokens, KVH, G, D, qk_scale,
+                      out_scale, signs, k8, chunk, scratch, scratch_bytes, out, out_f32, workspace, stream, false);
+}
+
+extern "C" int hkv_selftest_prefill_timeout(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd,
+                                            const void* vsf, const int64_t strides[6], int PS, const int32_t* block_tables,
+                                            int n_tables, int MP, const int32_t* rows, int n_rows, int n_tokens, int KVH, int G,
+                                            int D, float qk_scale, float out_scale, const float* signs, int k8, int64_t chunk,
+                                            void* scratch, size_t scratch_bytes, void* out, int out_f32, void* workspace,
+                                            void* stream) {
+  return prefill_impl(q, q_f16, kd, ksf, vd, vsf, strides, PS, block_tables, n_tables, MP, rows, n_rows, n_tokens, KVH, G, D, qk_scale,
+                      out_scale, signs, k8, chunk, scratch, scratch_bytes, out, out_f32, workspace, stream, true);
 }

@@ -254,7 +254,8 @@ def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, K
     contiguous; out (>= NT, HQ, D) bf16 or fp32 contiguous, other rows untouched.
     out = softmax(q k^T * qk_scale) v * out_scale, the cached values taken without their global scales. `chunk` bounds
     the tokens that are held as 16-bit operands at a time; the scratch comes from torch's allocator. signs as in
-    decode_ragged. The reference's counterpart is backend.py:438-543."""
+    decode_ragged. A device-side wait that ran out shows in workspace_status(workspace), without one in
+    workspace_status(None). The reference's counterpart is backend.py:438-543."""
     rc = (_lib._host or _lib.host()).prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, KVH, out,
                                              chunk, signs, k8, workspace)
     if rc is not None:
@@ -312,8 +313,12 @@ def set_option(option: int, value: int) -> None:
 
 
 def workspace_status(workspace) -> int:
-    """device status word of the last launches (0 = ok); synchronises, for tests and debugging"""
+    """device status word of the last launches (0 = ok); synchronises, for tests and debugging. None: that of the calls on the
+    current device that had no workspace"""
     st = C.c_int(0)
+    if workspace is None:
+        _lib.check(_lib.load().hkv_decode_noalloc_status(C.byref(st), _stream()), "hkv_decode_noalloc_status")
+        return int(st.value)
     with torch.cuda.device(workspace.device):
         rc = _lib.load().hkv_workspace_status(_ptr(workspace), C.byref(st), _stream())
     _lib.check(rc, "hkv_workspace_status")

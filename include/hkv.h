@@ -132,8 +132,8 @@ int hkv_decode_noalloc(const void* q, const void* kd, const void* ksf, const voi
                        float v_scale, const float* gk, const float* gv, int splits, void* out, void* stream);
 
 /*
- * Status word of the built-in scratch of hkv_decode_noalloc on the current device (HKV_OK or HKV_ERR_DEVICE_WAIT), read
- * and cleared like hkv_workspace_status does for a caller's workspace; synchronises the stream. No counterpart in the
+ * Status word of the built-in scratch of hkv_decode_noalloc on the current device (HKV_OK or HKV_ERR_DEVICE_WAIT), which
+ * hkv_prefill without a workspace sets too; read and cleared like hkv_workspace_status does for a caller's workspace; synchronises the stream. No counterpart in the
  * reference.
  */
 int hkv_decode_noalloc_status(int* status, void* stream);
@@ -238,7 +238,8 @@ int hkv_selftest_wait_timeout(void* workspace, int64_t cycles, void* stream);
  *                   launches end
  *   out             (>= n_tokens, KVH * G, D) bf16 or (out_f32) fp32, contiguous, 16-byte aligned; only the rows' tokens
  *                   are written: softmax(q k^T * qk_scale) v * out_scale, without global scales beyond these two
- *   workspace       NULL or a decode workspace, whose status word a bounded wait that ran out would set
+ *   workspace       a decode workspace, whose status word a bounded wait that ran out would set (hkv_workspace_status), or
+ *                   NULL: that of the array inside the library (hkv_decode_noalloc_status)
  * hkv_prefill_scratch_bytes returns 0 for arguments that hkv_prefill refuses.
  */
 size_t hkv_prefill_scratch_bytes(const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, int64_t chunk,
@@ -248,6 +249,16 @@ int hkv_prefill(const void* q, int q_f16, const void* kd, const void* ksf, const
                 int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale, float out_scale,
                 const float* signs, int k8, int64_t chunk, void* scratch, size_t scratch_bytes, void* out, int out_f32,
                 void* workspace, void* stream);
+/*
+ * Self-test of the path on which the prefill's attention kernel gives up: the same call, but every CTA stops fetching after
+ * three stages and its waits run out after a millisecond. The launch ends, the status word reads HKV_ERR_DEVICE_WAIT and the
+ * output of contexts of more than a few hundred tokens is undefined.
+ */
+int hkv_selftest_prefill_timeout(const void* q, int q_f16, const void* kd, const void* ksf, const void* vd, const void* vsf,
+                                 const int64_t strides[6], int PS, const int32_t* block_tables, int n_tables, int MP,
+                                 const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, float qk_scale,
+                                 float out_scale, const float* signs, int k8, int64_t chunk, void* scratch,
+                                 size_t scratch_bytes, void* out, int out_f32, void* workspace, void* stream);
 
 /*
  * Self-test of the narrow-float conversions the kernels stand on, no counterpart in the reference (whose CPU tests

@@ -7,6 +7,7 @@ import torch
 
 import synth
 from cases import bf16_tensor
+from horizon_kernels_b200 import _lib
 from horizon_kernels_b200 import kernels as K
 from horizon_kernels_b200 import layout as Lt
 from oracle import kvfp4 as O
@@ -238,3 +239,33 @@ def test_non_finite_queries_and_scales(D, ql, L, chunk):
     assert got[hit].isnan().all() and torch.equal(got[~hit], want[~hit]) and torch.isfinite(want.float()).all()
     for a, b in ((float("nan"), 1.0), (1.0, float("nan"))):
         assert call(q, a, b).isnan().all(), (a, b)
+
+
+@pytest.mark.parametrize("own", [True, False])
+@pytest.mark.parametrize("D,chunk", [(128, 65536), (256, 65536), (128, 256)])
+def test_a_wait_that_runs_out_ends_the_launch_and_is_reported(D, chunk, own):
+    """the give-up path of the attention kernel: every CTA stops fetching early, its waits run out after a millisecond, the
+    launches end and the status word of the workspace (without one: of the library's own) says so, once; the same call then
+    works, to the bit"""
+    import ctypes as C
+    KVH, G, ql, L = 2, 4, 700, 1500
+    k, v = torch.randn(2, L, KVH, D, device="cuda")
+    flat, strides, bt = filled(KVH, D, L, k, v, 0.01)
+    q = torch.randn(ql, KVH * G, D, device="cuda").to(torch.bfloat16)
+    ws = K.alloc_workspace(1, KVH, G, D) if own else None
+    want, out = torch.zeros_like(q), torch.zeros_like(q)
+    K.prefill(q, flat, strides, 16, bt, [(0, 0, ql, L)], D ** -0.5, 1.0, KVH, want, chunk=chunk, workspace=ws)
+    assert K.workspace_status(ws) == 0
+    lib, p = _lib.load(), lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    host_rows = (C.c_int32 * 4)(0, 0, ql, L)
+    nb = lib.hkv_prefill_scratch_bytes(host_rows, 1, ql, KVH, G, D, chunk, 0)
+    scratch = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    call = lambda f: f(p(q), 0, *(p(t) for t in flat), (C.c_int64 * 6)(*strides), 16, p(bt), *bt.shape, host_rows, 1, ql, KVH, G, D,  # noqa: E731
+                       D ** -0.5, 1.0, None, 0, chunk, p(scratch), nb, p(out), 0, p(ws) if own else None,
+                       C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert call(lib.hkv_selftest_prefill_timeout) == 0
+    assert K.workspace_status(ws) == -8                  # HKV_ERR_DEVICE_WAIT, cleared by the read
+    assert K.workspace_status(ws) == 0
+    assert call(lib.hkv_prefill) == 0
+    assert K.workspace_status(ws) == 0
+    assert torch.equal(out, want)
