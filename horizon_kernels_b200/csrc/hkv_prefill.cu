@@ -960,7 +960,8 @@ __global__ void __launch_bounds__(256) merge_kernel(const __grid_constant__ Pref
   const int end = (max(1, min(r.L, r.L - r.ql + min(r.ql, (t.rt + 1) * p.tok))) + kKeys - 1) / kKeys;
   if (state && end > p.kt_hi) {
     float* so = p.state_o + st_row * D + ch;
-    __syncwarp(__activemask());                           // a row's lanes have read its state
+    // a row's lanes (they agree on the return above) have read its state
+    __syncwarp(LPR == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16));
 #pragma unroll
     for (int k = 0; k < 8; ++k) so[k] = acc[k];
     if (ch == 0) {
