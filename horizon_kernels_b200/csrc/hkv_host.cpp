@@ -206,7 +206,7 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (q->scalar_type() != at::kBFloat16 || (out->scalar_type() != at::kBFloat16 && !out_f32) || q->dim() != 3 || out->dim() != 3 ||
         out->size(1) != q->size(1) || out->size(2) != q->size(2) || out->size(0) < q->size(0) || !q->is_contiguous() ||
         !out->is_contiguous() || !on(*out, dev) || !on(*bt, dev) || bt->scalar_type() != at::kInt || bt->dim() != 2 ||
-        !bt->is_contiguous() || (ws && !on(*ws, dev)))
+        !bt->is_contiguous() || (ws && (!on(*ws, dev) || ws->nbytes() < 64)))
       Py_RETURN_NONE;
     const int64_t B = bt->size(0), MP = bt->size(1), NT = q->size(0), HQ = q->size(1), D = q->size(2);
     if (HQ % KVH || B > INT32_MAX || MP > INT32_MAX || NT > INT32_MAX || HQ > INT32_MAX || D > INT32_MAX ||

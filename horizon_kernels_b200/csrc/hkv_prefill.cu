@@ -1133,7 +1133,7 @@ static int prefill_impl(const void* q, int q_f16, const void* kd, const void* ks
   if (PS < 1) return HKV_ERR_UNSUPPORTED;
   if (((uintptr_t)kd | (uintptr_t)vd | (uintptr_t)strides[0] | (uintptr_t)strides[1] | (uintptr_t)strides[2]) & 7) return HKV_ERR_ALIGN;
   if (k8 && (((uintptr_t)kd | (uintptr_t)strides[0] | (uintptr_t)strides[1] | (uintptr_t)strides[2]) & 15)) return HKV_ERR_ALIGN;
-  if (((uintptr_t)q | (uintptr_t)out) & 15 || ((uintptr_t)scratch & 255)) return HKV_ERR_ALIGN;
+  if (((uintptr_t)q | (uintptr_t)out) & 15 || (((uintptr_t)scratch | (uintptr_t)workspace) & 255)) return HKV_ERR_ALIGN;
   for (int i = 0; i < n_rows; ++i)
     if (rows[4 * i] >= n_tables || (int64_t)rows[4 * i + 3] > (int64_t)MP * PS) return HKV_ERR_RANGE;
   const int ct = chunk_tiles_of(chunk);

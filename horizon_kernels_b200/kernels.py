@@ -13,6 +13,7 @@ from . import _lib
 from .layout import flat_views  # noqa: F401  (re-exported: part of the reference's API)
 
 LOG2E = 1.4426950408889634
+WORKSPACE_HEADER_BYTES = 64        # the status word and its padding, at the start of every workspace
 _SMS = {}
 
 
@@ -287,12 +288,16 @@ def prefill(query, flat, strides, PS, block_tables, rows, qk_scale, out_scale, K
             raise ValueError(f"prefill row {(row, q0, q1, L)} of {B} requests and {NT} query tokens")
     _need_cuda(query, block_tables, out, *flat)
     _check_signs(signs, D)
+    if workspace is not None:
+        _need_cuda(workspace)
+        if workspace.device != query.device or workspace.nbytes < WORKSPACE_HEADER_BYTES:
+            raise ValueError("workspace must come from alloc_workspace on the query's device")
     n = len(rows)
     host_rows = (C.c_int32 * (4 * n))(*[int(x) for r in rows for x in r])
     lib = _lib.load()
-    nb = int(lib.hkv_prefill_scratch_bytes(host_rows, n, NT, KVH, HQ // KVH, D, int(chunk), int(signs is not None)))
     kd, ksf, vd, vsf = flat
-    with torch.cuda.device(query.device):
+    with torch.cuda.device(query.device):                # (the scratch grows with that device's SMs)
+        nb = int(lib.hkv_prefill_scratch_bytes(host_rows, n, NT, KVH, HQ // KVH, D, int(chunk), int(signs is not None)))
         scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device=query.device)
         rc = lib.hkv_prefill(_ptr(query), int(query.dtype == torch.float16), _ptr(kd), _ptr(ksf), _ptr(vd), _ptr(vsf),
                              (C.c_int64 * 6)(*strides), int(PS), _ptr(block_tables), B, MP, host_rows, n, NT, KVH, HQ // KVH,

@@ -238,7 +238,7 @@ int hkv_selftest_wait_timeout(void* workspace, int64_t cycles, void* stream);
  *                   launches end
  *   out             (>= n_tokens, KVH * G, D) bf16 or (out_f32) fp32, contiguous, 16-byte aligned; only the rows' tokens
  *                   are written: softmax(q k^T * qk_scale) v * out_scale, without global scales beyond these two
- *   workspace       a decode workspace, whose status word a bounded wait that ran out would set (hkv_workspace_status), or
+ *   workspace       a decode workspace (256-byte aligned), whose status word a bounded wait that ran out would set (hkv_workspace_status), or
  *                   NULL: that of the array inside the library (hkv_decode_noalloc_status)
  * hkv_prefill_scratch_bytes returns 0 for arguments that hkv_prefill refuses.
  */

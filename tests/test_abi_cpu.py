@@ -107,6 +107,42 @@ def test_dequant_rejects_misuse(lib):
     assert call(start=60, n=8) == -6                           # positions beyond the 4-page block-table row
 
 
+def test_prefill_rejects_misuse(lib):
+    one = C.c_void_p(0x1000)
+    base = dict(q=one, f16=0, kd=one, ksf=one, vd=one, vsf=one, st=_strides(18432, 72, 1152, 18432, 72, 1152), PS=16, bt=one, B=2,
+                MP=8, rows=(C.c_int32 * 4)(1, 0, 40, 100), n=1, NT=40, KVH=8, G=4, D=128, signs=None, k8=0, chunk=65536,
+                scratch=one, nb=1 << 40, out=one, ws=one)
+
+    def call(**kw):
+        a = dict(base, **kw)
+        return lib.hkv_prefill(a["q"], a["f16"], a["kd"], a["ksf"], a["vd"], a["vsf"], a["st"], a["PS"], a["bt"], a["B"], a["MP"],
+                               a["rows"], a["n"], a["NT"], a["KVH"], a["G"], a["D"], 0.088, 1.0, a["signs"], a["k8"], a["chunk"],
+                               a["scratch"], a["nb"], a["out"], 0, a["ws"], None)
+
+    def row(*v):
+        return (C.c_int32 * 4)(*v)
+    assert call(n=0) == 0                                    # nothing to do, nothing launched
+    assert call(n=-1) == -6
+    for name in ("q", "kd", "ksf", "vd", "vsf", "bt", "scratch", "out", "rows"):
+        assert call(**{name: None}) == -1, name
+    for name, at in (("q", 0x1008), ("out", 0x1008), ("kd", 0x1004), ("vd", 0x1004), ("scratch", 0x1080), ("ws", 0x1010)):
+        assert call(**{name: C.c_void_p(at)}) == -2, name
+    assert call(st=_strides(18432, 70, 1152, 18432, 72, 1152)) == -2
+    assert call(k8=1, D=256, kd=C.c_void_p(0x1008)) == -2    # FP8 keys are read 16 bytes at a time
+    assert call(D=64) == call(G=129) == call(KVH=0) == call(KVH=1025) == call(PS=0) == -3
+    assert call(k8=1) == -3                                  # the FP8-key slot exists at head_dim 256
+    assert call(signs=one, f16=1) == call(signs=one, k8=1, D=256) == -3
+    for r in (row(-1, 0, 40, 100), row(2, 0, 40, 100), row(1, -1, 40, 100), row(1, 7, 7, 100), row(1, 0, 41, 100),
+              row(1, 0, 40, 0), row(1, 0, 40, 129)):         # table row, query tokens, context, positions beyond the table
+        assert call(rows=r) == -6, tuple(r)
+    need = lib.hkv_prefill_scratch_bytes(base["rows"], 1, 40, 8, 4, 128, 65536, 0)
+    assert need > 0 and call(nb=need - 1) == -5
+    assert lib.hkv_prefill_scratch_bytes(base["rows"], 1, 40, 8, 4, 128, 65536, 1) > need
+    for a in ((None, 1, 40, 8, 4, 128), (base["rows"], 0, 40, 8, 4, 128), (base["rows"], 1, 39, 8, 4, 128),
+              (base["rows"], 1, 40, 8, 129, 128), (base["rows"], 1, 40, 8, 4, 96)):
+        assert lib.hkv_prefill_scratch_bytes(*a, 65536, 0) == 0, a
+
+
 def test_set_option_codes(lib):
     assert lib.hkv_set_option(99, 1) == -3
     assert lib.hkv_set_option(1, 2) == -6

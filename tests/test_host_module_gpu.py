@@ -31,8 +31,8 @@ def _decode(s, out, PS=PS, scale=0.05, **kw):
                            1, out, s["ws"], **kw)
 
 
-def _prefill(s, out, rows, PS=PS, chunk=65536):
-    return K.prefill(s["q"], s["flat"], s["strides"], PS, s["bt"], rows, 0.05, 1.0, KVH, out, chunk=chunk)
+def _prefill(s, out, rows, PS=PS, chunk=65536, **kw):
+    return K.prefill(s["q"], s["flat"], s["strides"], PS, s["bt"], rows, 0.05, 1.0, KVH, out, chunk=chunk, **kw)
 
 
 class AnInt(int):
@@ -80,6 +80,12 @@ def test_refusals_are_the_python_ones():
         _prefill(s, out, [(3, 0, 2, 100)])
     with pytest.raises(ValueError):
         _prefill(s, out, [(0, 1, 4, 100)])
+    with pytest.raises(RuntimeError):                    # the status word is written by the kernel
+        _prefill(s, out, [(0, 0, 2, 100)], workspace=s["ws"].cpu())
+    with pytest.raises(ValueError, match="workspace"):
+        _prefill(s, out, [(0, 0, 2, 100)], workspace=s["ws"][:32])
+    with pytest.raises(_lib.HkvError):
+        _prefill(s, out, [(0, 0, 2, 100)], workspace=s["ws"][4:])
     assert not out.any()
 
 
