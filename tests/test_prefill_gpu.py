@@ -131,21 +131,25 @@ def test_graph_capture_and_repeat():
     assert torch.equal(out, eager)
 
 
-def filled(KVH, D, L, k, v, gk, PS=16, n_req=1):
-    """head-major cache of n_req requests of L tokens with the given keys and values, (flat, strides), block tables"""
+def filled(KVH, D, L, k, v, gk, PS=16, nhd=False, k8=False, signs=None):
+    """cache of one request of L tokens with the given keys and values: (flat, strides), block table"""
     dev = torch.device("cuda")
     per = (L + PS - 1) // PS
-    cache = Lt.alloc_cache(per * n_req + 2, PS, KVH, D, device=dev, fill=0x7F)
-    flat, strides = Lt.flat_views(*Lt.slot_views(cache, KVH, D))
-    bt = torch.randperm(per * n_req, device=dev).to(torch.int32).view(n_req, per)
+    heads, slot = (KVH, Lt.k8_slot_bytes(D)) if k8 else (2 * KVH, Lt.slot_bytes(D))
+    if nhd:
+        cache = torch.full((per + 2, PS, heads, slot), 0x7F, dtype=torch.uint8, device=dev).permute(0, 2, 1, 3)
+    else:
+        cache = torch.full((per + 2, heads, PS, slot), 0x7F, dtype=torch.uint8, device=dev)
+    flat, strides = Lt.k8_flat_views(*Lt.k8_views(cache, D)) if k8 else Lt.flat_views(*Lt.slot_views(cache, KVH, D))
+    bt = torch.randperm(per, generator=torch.Generator().manual_seed(L)).to(torch.int32).view(1, per).to(dev)
     pos = torch.arange(L, device=dev)
-    slots = (bt[:, pos // PS].long() * PS + pos % PS).reshape(-1)
+    slots = bt[0, pos // PS].long() * PS + pos % PS
     one = torch.ones(KVH, device=dev)
-    K.write(k.to(torch.bfloat16), v.to(torch.bfloat16), flat, strides, PS, slots, gk * one, one)
+    K.write(k.to(torch.bfloat16), v.to(torch.bfloat16), flat, strides, PS, slots, gk * one, one, signs=signs, k8=k8)
     return flat, strides, bt
 
 
-def attend64(q, flat, strides, PS, bt, rows, KVH, sm, f16_probabilities=False):
+def attend64(q, flat, strides, PS, bt, rows, KVH, sm, f16_probabilities=False, k8=False):
     """per (token, head) in 64 bits: the output, sum_j w_j |v_j|, and the largest score (log2) of every 128 keys; optionally
     with the probabilities rounded to f16 under the row's exact maximum before the value product"""
     NT, HQ, D = q.shape
@@ -154,7 +158,7 @@ def attend64(q, flat, strides, PS, bt, rows, KVH, sm, f16_probabilities=False):
     tops = {}
     for b, q0, q1, L in rows:
         kk, vv = (torch.empty(L, KVH, D, dtype=torch.float16, device=q.device) for _ in range(2))
-        K.dequant_tokens(flat, strides, PS, bt[b].contiguous(), 0, L, kk, vv)
+        K.dequant_tokens(flat, strides, PS, bt[b].contiguous(), 0, L, kk, vv, k8=k8)
         ql = q1 - q0
         hidden = torch.arange(L, device=q.device)[None] >= torch.arange(L - ql + 1, L + 1, device=q.device).repeat_interleave(G)[:, None]
         for h in range(KVH):
@@ -269,3 +273,41 @@ def test_a_wait_that_runs_out_ends_the_launch_and_is_reported(D, chunk, own):
     assert call(lib.hkv_prefill) == 0
     assert K.workspace_status(ws) == 0
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("chunk", [65536, 384])
+@pytest.mark.parametrize("KVH,G,D,PS", [(2, 4, 128, 16), (3, 2, 128, 32), (1, 8, 128, 64), (2, 8, 256, 16), (3, 4, 256, 64)])
+def test_positions_outermost_pages(KVH, G, D, PS, chunk):
+    """vLLM's other page order: the bits of head-major pages of the same tokens (odd kv head counts put token rows off the
+    16-byte grid at head_dim 128)"""
+    ql, L = 150, 1300
+    g = torch.Generator(device="cuda").manual_seed(D + PS)
+    k, v = torch.randn(2, L, KVH, D, generator=g, device="cuda")
+    q = torch.randn(ql, KVH * G, D, generator=g, device="cuda").to(torch.bfloat16)
+    got = []
+    for nhd in (False, True):
+        flat, strides, bt = filled(KVH, D, L, k, v, 0.01, PS, nhd=nhd)
+        got.append(K.prefill(q, flat, strides, PS, bt, [(0, 0, ql, L)], 0.01 * D ** -0.5, 1.0, KVH, torch.zeros_like(q), chunk=chunk))
+    assert torch.equal(got[0], got[1]) and got[0].any()
+
+
+@pytest.mark.parametrize("chunk", [65536, 1000, 384])
+@pytest.mark.parametrize("D,option", [(128, "rotated"), (256, "rotated"), (256, "k8"), (128, "f16"), (256, "f16")])
+def test_options_over_chunks(D, option, chunk):
+    """rotated keys, FP8 keys and f16 queries in one and in several chunks, every element against 64 bits"""
+    KVH, G, ql, L = 2, 4, 150, 1700
+    g = torch.Generator(device="cuda").manual_seed(D + ql)
+    k, v = torch.randn(2, L, KVH, D, generator=g, device="cuda")
+    k[:, :, [3, D // 2 + 3]] *= 20.0
+    q = torch.randn(ql, KVH * G, D, generator=g, device="cuda").to(torch.float16 if option == "f16" else torch.bfloat16)
+    signs = K.hadamard_signs(D, device="cuda") if option == "rotated" else None
+    k8 = option == "k8"
+    gk = 0.25 if k8 else 0.04
+    flat, strides, bt = filled(KVH, D, L, k, v, gk, k8=k8, signs=signs)
+    rows, sm, out = [(0, 0, ql, L)], D ** -0.5 * gk, torch.zeros(ql, KVH * G, D, device="cuda")
+    K.prefill(q, flat, strides, 16, bt, rows, sm, 1.0, KVH, out, chunk=chunk, signs=signs, k8=k8)
+    q64 = q if signs is None else K.rotate(q, signs).to(torch.bfloat16)
+    want, absv, _ = attend64(q64, flat, strides, 16, bt, rows, KVH, sm, k8=k8)
+    # as in test_maxima_that_rise_in_every_tile
+    bound = absv * (2.0 ** -11 + 2.0 ** -12) + L * 2.0 ** -25 * float(v.abs().max()) * 2
+    assert ((out.double() - want).abs() <= bound).all()

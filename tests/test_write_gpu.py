@@ -58,7 +58,10 @@ def kv_tokens(seed, NT, KVH, D, kind):
 @pytest.mark.parametrize("D,KVH,PS", [(128, 8, 16), (256, 2, 16), (256, 4, 64)])
 @pytest.mark.parametrize("kind", ["random", "outlier", "edge"])
 def test_write_matches_oracle(D, KVH, PS, kind):
-    for NT in (1, 7, 300):
+    # 60 tokens hold every edge row and go four lanes to a block; `line` is the last count that does, the next goes one lane
+    # to a block, as 300 do
+    line = 19000 // (2 * KVH * D // 16)
+    for NT in (1, 7, 60, line, line + 1, 300):
         NP = (NT + PS - 1) // PS + 3
         slots = synth.permutation(5 + NT, NP * PS)[:NT].astype(np.int64)
         slots[synth.uniform(6 + NT, NT) < 0.1] = -1
@@ -82,7 +85,7 @@ def test_write_matches_oracle(D, KVH, PS, kind):
 @pytest.mark.parametrize("kind", ["edge", "outlier"])
 @pytest.mark.parametrize("D,KVH", [(128, 8), (256, 2)])
 def test_large_launch_one_lane_per_block_matches_oracle(D, KVH, kind):
-    """more than 4096 tokens: the launch gives every block to ONE lane, which scores the four scale candidates itself
+    """many more than 19000 blocks: the launch gives every block to ONE lane, which scores the four scale candidates itself
     (packed fp32 pairs, quotients by multiply-adds) and falls back to IEEE divisions for zero blocks, tiny and huge
     scales; the edge rows (zeros, 1e-30, 1e30, -0.0, exact ties) go through both paths. The edge tokens are repeated
     across the launch so that whole warps and single lanes of a warp meet them."""
