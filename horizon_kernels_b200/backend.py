@@ -26,7 +26,7 @@ from .layout import flat_views, k8_flat_views, k8_slot_bytes, k8_views, slot_byt
 
 HEAD_SIZES = (128, 256)
 PAGE_SIZES = (16, 32, 64)
-MAX_ROWS = 64                     # query rows per kv head, G * (1 + draft tokens): eight per pass over the cache
+MAX_ROWS = 64                     # query rows per kv head, G * (1 + draft tokens): sixteen (or eight) per pass over the cache
 _STATE = {}                       # per device: decode workspace
 
 

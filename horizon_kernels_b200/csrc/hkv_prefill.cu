@@ -11,9 +11,9 @@
 // Replaces the reference's library attention over dequantised tokens (backend.py:438-543).
 //
 // Layer steps on a B200 (write launch included): a fresh prompt of 6144 tokens, 32 query heads over 8 kv heads, head_dim 128:
-// 361 us (tile 12, attend about 295, merge 7) against 16.5 ms with torch matmuls and eager softmax passes, whose fp32 score
-// matrices went through memory. 2048 tokens over 30000 cached, 16 heads over 2, head_dim 256: 0.85 ms, at which the board
-// draws its 1000 W and the clock falls to 1.6 GHz (1.25 PFLOP/s; a plain bf16 GEMM sustains 1.37), against 15.0 ms.
+// 372 us against 16.5 ms with torch matmuls and eager softmax passes, whose fp32 score matrices went through memory. 2048
+// tokens over 30000 cached, 16 heads over 2, head_dim 256: 0.91 ms (1.14 PFLOP/s; a plain bf16 GEMM sustains 1.37 at the
+// board's 1000 W) against 15.0 ms.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -404,7 +404,7 @@ __device__ __forceinline__ void store_out(const PrefillParams& p, long long elem
 // Why so: a score tile is 1024 clocks of exponentials (ex2: 16 per clock and SM) and twice that again in latencies (loads
 // from tensor memory, barriers, contention) before its value product can start, while the tensor pipe needs 1024 clocks
 // (head_dim 128) or 2048 for both products. Two 128-row sub-tiles with one score buffer each left the tensor pipe idle 45 %
-// of the time (3590 clocks for both against 2048; here 1450 a tile) and 9000 clocks between pieces (here about 3000; short
+// of the time (3590 clocks for both against 2048; here 1450 a tile before the maximum was exact) and 9000 clocks between pieces (here about 3000; short
 // prompts gain most, a step of four prompts with 48 decode requests went from 128 to 117 us); 64-key steps with two buffers
 // each paid twice for the score product, which reads its 128 query rows from shared memory whatever the number of keys.
 // The 16-bit probabilities go over the scores they came from. A thread tells the next tile's thread of its row the running
@@ -412,8 +412,9 @@ __device__ __forceinline__ void store_out(const PrefillParams& p, long long elem
 // the wait for the value product before it then passes behind the exponentials. The maximum is the exact one: the largest
 // probability is 1 and loses nothing to the rounding to f16. One that lags by up to 2^14 hardly ever rescales, but its
 // largest probability is any number: the error against 64 bits (before the output's own rounding) was 1.9e-4 where this has
-// 6.5e-5 (a prompt of 6144 tokens, head_dim 128: 324 us either way; 518 us with the rescaling before the exponentials) and
-// 2.0e-4 where this has 8.3e-5 (2048 tokens over 30000, head_dim 256: 735 us there, 770 here).
+// 6.5e-5 (a prompt of 6144 tokens, head_dim 128) and 2.0e-4 where this has 8.3e-5 (2048 tokens over 30000, head_dim 256);
+// the torch path before had 8.0e-5 and 1.06e-4. With the lag the steps took 361 and 862 us, now 372 and 915; with the rescaling
+// before the exponentials 1.6 and 1.3 times as long.
 // A walk over the CTA's key tiles, piece by piece. A step to the next row tile of a request costs a few instructions: every
 // role takes it at every piece, two of them in a single thread.
 struct Tiles {
@@ -814,8 +815,9 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
               if (i >= rel) s0[i] = 0xff800000u;
           }
         };
-        // (rolled loops, and no register to spare: unrolled, the code of all roles leaves the instruction cache, and a
-        // spilled register costs an L2 access, since the L1 cache is all shared memory; each made the launch 8 to 15 % longer)
+        // (rolled loops, and no register to spare: unrolled, the code of all roles leaves the instruction cache, and a register
+        // spilled in here costs an L2 access, since the L1 cache is all shared memory; each made the launch 8 to 15 % longer. At
+        // head_dim 256 the compiler spills 24 bytes of the 128 registers that 512 threads leave, in all)
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           load(c);
@@ -859,7 +861,7 @@ __global__ void __launch_bounds__(PfShape<D>::THREADS, 1) attend_kernel(const __
         }
         if (__any_sync(0xffffffffu, al_o != 1.0f)) {
           // the output of the tiles before this one, all of whose value products must have been added first; 64 columns at a
-          // time and in packed pairs (32 at a time, one by one: 787 us where this takes 770, head_dim 256)
+          // time and in packed pairs (32 at a time and one by one, a step at head_dim 256 took 2 % longer)
           ok = all_wait(o_done0 + 8 * before, (g - 1) / SETS);
           if (!ok) {
             tc_wait_st();

@@ -222,7 +222,7 @@ __device__ __forceinline__ void score(const f32x2 (&AX)[8], float amax, float sc
   }
 }
 
-// LPB lanes own one block of 16 consecutive channels of one (token, kv head, side). LPB = 1 (more than about 150 tokens):
+// LPB lanes own one block of 16 consecutive channels of one (token, kv head, side). LPB = 1 (more than 19000 blocks, 148 tokens of 8 x 128):
 // the lane reads the block's 32 bytes, scores the four scale candidates one after the other, keeps the codes of the
 // best one and stores 8 code bytes and the scale byte: consecutive lanes cover consecutive blocks, so a warp reads 1 KB
 // and stores 256 B contiguous. LPB = 4 (few tokens, latency matters): the four lanes of a quad read the same block,
@@ -646,6 +646,7 @@ static int write_impl(const void* key, const void* val, int64_t ks0, int64_t ks1
   // sooner), one lane for more, and whenever the keys are rotated. The line lies where the quads start to queue on the SMs'
   // pipes. 8 kv heads x 128, with the search, back to back: 16384 blocks (128 tokens) 3.0 us with quads, 3.1 with single
   // lanes; 32768 blocks 4.2 / 3.2; 262144 blocks (2048 tokens) 16.7 / 9.0. 2 x 256: 16384 blocks 2.9 / 3.2; 32768 4.2 / 3.2.
+  // Without the search (in a captured chain of launches): 18944 blocks 2.1 with quads, 20480 blocks 2.3 / 1.9; 262144 11.7 / 4.0.
   const int lpb = (n_slots * (2ll * KVH * (D / 16)) <= 19000 && !signs && !k8) ? 4 : 1;
   const int threads = 256;
   const long long lanes = n_slots * (2ll * KVH * (D / 16)) * lpb;

@@ -84,7 +84,8 @@ size_t hkv_decode_workspace_bytes(int B, int KVH, int G, int D, int qlmax);
  *   block_tables : int32 (B, MP); seq_lens int32 (B); query_start_loc int32 (B + 1)
  *   requests with 0 or more than qlmax query tokens are skipped and their output rows left untouched
  *   out          : bf16 (>= n_tokens, KVH*G, D) contiguous
- * A pass over the cache serves 8 query rows per kv head, or 16 at head_dim 128 over head-major slot pages (the reference
+ * A pass over the cache serves 8 query rows per kv head, or 16 over head-major slot pages (at head_dim 256 where the
+ * workspace, sized by hkv_decode_workspace_bytes for these rows, holds their partials; the reference
  * serves up to 32 rows in one launch, backend.py:237). G * qlmax within one pass is one launch. Up to 64 rows are
  * accepted: the call then makes ceil(G * qlmax / rows per pass) launches.
  */
@@ -238,8 +239,8 @@ int hkv_selftest_wait_timeout(void* workspace, int64_t cycles, void* stream);
  *                   launches end
  *   out             (>= n_tokens, KVH * G, D) bf16 or (out_f32) fp32, contiguous, 16-byte aligned; only the rows' tokens
  *                   are written: softmax(q k^T * qk_scale) v * out_scale, without global scales beyond these two
- *   workspace       a decode workspace (256-byte aligned), whose status word a bounded wait that ran out would set (hkv_workspace_status), or
- *                   NULL: that of the array inside the library (hkv_decode_noalloc_status)
+ *   workspace       a decode workspace (256-byte aligned), whose status word a bounded wait that ran out would set
+ *                   (hkv_workspace_status), or NULL: that of the array inside the library (hkv_decode_noalloc_status)
  * hkv_prefill_scratch_bytes returns 0 for arguments that hkv_prefill refuses.
  */
 size_t hkv_prefill_scratch_bytes(const int32_t* rows, int n_rows, int n_tokens, int KVH, int G, int D, int64_t chunk,

@@ -66,9 +66,9 @@ def test_update_then_forward_matches_oracle(KVH, G, D, PS, nhd):
 @pytest.mark.parametrize("KVH,G,D,PS", [(8, 4, 128, 16), (2, 8, 256, 16)])
 def test_mixed_step_with_prefill_rows(KVH, G, D, PS, chunk, pf16, monkeypatch):
     """a step with decode rows (1 query token) and prefill rows over a cached prefix (37 and 300 query tokens): the
-    decode kernel serves the former and leaves the latter untouched, the dequantise + attention path serves the latter;
+    decode kernel serves the former and leaves the latter untouched, the prefill kernels serve the latter;
     both against the oracle with the reference's causal window"""
-    # (prefill contexts are dequantised in chunks merged by a running log-sum-exp: the small chunk sizes cut the 700-token
+    # (prefill contexts become 16-bit operands in chunks of at least 128 tokens: the small chunk sizes cut the 700-token
     # context into several chunks that do not end on page boundaries; compute dtype fp16 or bf16)
     monkeypatch.setenv("HORIZON_KVFP4_CHUNK", chunk)
     monkeypatch.setenv("HORIZON_KVFP4_PF16", pf16)
@@ -110,7 +110,7 @@ def test_mixed_step_with_prefill_rows(KVH, G, D, PS, chunk, pf16, monkeypatch):
             dec[int(c["qsl"][b])] = True
     got[torch.from_numpy(dec).to(dev)] /= vscale
     assert_close(got[torch.from_numpy(dec).to(dev)], want[dec], "decode rows")
-    # prefill rows go through a library bf16 attention (probabilities rounded to bf16): the reference's own gate,
+    # prefill rows have probabilities rounded to f16 and the output rounded to bf16: the reference's own gate,
     # relative L2, holds; the absolute error scales with the outputs, which reach the values' outliers here
     mx, mn, rl = errors(got[torch.from_numpy(~dec).to(dev)], want[~dec])
     assert rl <= 2.5e-3 and mn <= 2e-3 and mx <= 6e-2, (mx, mn, rl)
@@ -118,7 +118,7 @@ def test_mixed_step_with_prefill_rows(KVH, G, D, PS, chunk, pf16, monkeypatch):
 
 def test_rotation_option_end_to_end(monkeypatch):
     """HORIZON_KVFP4_HAD=1: do_kv_cache_update writes rotated keys, forward rotates the queries of decode rows inside the
-    kernel and of prefill rows in torch; both against fp64 attention of rotate_q(q) over the rotated cache"""
+    kernel and of prefill rows in a launch of their own; both against fp64 attention of rotate_q(q) over the rotated cache"""
     monkeypatch.setenv("HORIZON_KVFP4_HAD", "1")
     from horizon_kernels_b200 import kernels as K
     KVH, G, D, PS = 4, 4, 128, 16

@@ -181,16 +181,15 @@ def test_long_context_split_and_combine():
     print("64k errors", mx, mn, rl)
 
 
-@pytest.mark.parametrize("D,KVH,G", [(128, 2, 4), (256, 1, 8), (128, 2, 8)])
-def test_every_sequence_split_over_three_or_more_partitions(D, KVH, G):
+@pytest.mark.parametrize("D,KVH,G,two", [(128, 2, 4, True), (256, 1, 8, False), (128, 2, 8, True), (256, 1, 8, True)])
+def test_every_sequence_split_over_three_or_more_partitions(D, KVH, G, two):
     """few long sequences on a grid that fills the GPU: every sequence is cut into many pieces (hundreds of partitions
     over 2 to 4 sequences), each merged inside the decode launch by whichever CTA finishes its last piece. The result
     must not depend on which CTA that is: three runs are bit-equal, the ticket counters are back at zero after every
     launch, and a cap on the partitions (`splits` 1 / 2 / 64, i.e. 1, 2 and up to 64 pieces per sequence) stays within
     the tolerance."""
     lens = [9000, 12345]
-    one_pass = 16 if D == 128 else 8                  # query rows per kv head a single pass serves
-    two = G * 2 <= one_pass                            # (group 8 x 2 tokens at head_dim 128: the sixteen-row kernel)
+    # (two query tokens at group 8: the sixteen-row kernel)
     c = build_decode_case(2210 + D + G, lens, KVH, G, D, 16, ql_list=[1, 2] if two else None)
     ref = oracle_decode(c, v_scale=0.5)
     qlmax = 2 if two else 1
@@ -250,7 +249,7 @@ def test_graph_replay_with_poisoned_output():
 @pytest.mark.parametrize("KVH,G,D,qls", [(2, 16, 128, [1, 1, 1]), (8, 4, 128, [4, 2, 4]), (2, 8, 256, [3, 1, 2]),
                                          (1, 12, 128, [5, 5, 1])])
 def test_more_than_eight_query_rows(KVH, G, D, qls):
-    """G * ql > 8 rows per kv head (large groups, several draft tokens): served eight rows per pass over the cache;
+    """G * ql > 8 rows per kv head (large groups, several draft tokens): served sixteen rows per pass over the cache;
     causal among the request's own query tokens; requests with fewer query tokens drop out of the later passes"""
     lens = [333, 40, 1500][:len(qls)]
     c = build_decode_case(2450 + G, lens, KVH, G, D, 16, ql_list=qls)
