@@ -21,6 +21,7 @@ from typing import ClassVar
 
 import torch
 
+from . import _lib
 from . import kernels as K
 from .layout import flat_views, k8_flat_views, k8_slot_bytes, k8_views, slot_bytes, slot_views
 
@@ -300,9 +301,16 @@ def _build_classes():
         # ---------------------------------------------------------------------------------------------- write
         def do_kv_cache_update(self, layer, key, value, kv_cache, slot_mapping):
             """reference backend.py:389-403"""
-            v = self._cache_views(kv_cache)
-            gk, gv = self._scales(layer, key.device)
+            gk, gv = (self._gk, self._gv) if self._gk is not None else self._scales(layer, key.device)
             D = self.head_size
+            # the usual arguments are taken as they are; through the views below the call takes half as long again
+            rc = (_lib._host or _lib.host()).layer_write(key, value, kv_cache, slot_mapping, gk, gv, D, self.search,
+                                                         self._rot(key.device) if self.had else None, self.k8)
+            if rc is not None:
+                if rc:
+                    _lib.check(rc, "hkv_write")
+                return
+            v = self._cache_views(kv_cache)
             k3 = key.view(key.shape[0], self.num_kv_heads, D) if key.dim() == 2 else key
             v3 = value.view(value.shape[0], self.num_kv_heads, D) if value.dim() == 2 else value
             K.write(k3, v3, v["flat"], v["strides"], v["PS"], slot_mapping, gk, gv, self.search,
@@ -319,15 +327,27 @@ def _build_classes():
             m = attn_metadata
             T = m.num_actual_tokens
             st = self._state(query.device)
+            gk, gv = (self._gk, self._gv) if self._gk is not None else self._scales(layer, query.device)
+            decode = m.has_decode and m.num_reqs > 0
+            if decode:                                # as in do_kv_cache_update: the usual arguments as they are
+                rc = (_lib._host or _lib.host()).layer_decode(
+                    query, kv_cache, m.block_table, m.seq_lens, m.query_start_loc, T, self.scale, float(layer._v_scale_float),
+                    gk, gv, m.qlmax, output, st["ws"], self.cps, self.num_heads, self.head_size,
+                    self._rot(query.device) if self.had else None, self.k8)
+                if rc is not None:
+                    if rc:
+                        _lib.check(rc, "hkv_decode")
+                    if not m.prefill_rows:
+                        return output
+                    decode = False
             v = self._cache_views(kv_cache)
-            gk, gv = self._scales(layer, query.device)
             q = query[:T]
             if q.dim() == 2:
                 q = q.view(T, self.num_heads, self.head_size)
             if not q.is_contiguous():
                 q = q.contiguous()
             out = output.view(output.shape[0], self.num_heads, self.head_size) if output.dim() == 2 else output
-            if m.has_decode and m.num_reqs > 0:
+            if decode:
                 K.decode_ragged(q, v["flat"], v["strides"], v["PS"], m.block_table, m.seq_lens, m.query_start_loc,
                                 self.scale, float(layer._v_scale_float), gk, gv, m.qlmax, out, st["ws"],
                                 splits=self.cps or None, signs=self._rot(q.device), k8=self.k8)

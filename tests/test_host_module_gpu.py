@@ -1,9 +1,12 @@
 """The native side of the host wrappers (csrc/hkv_host.cpp) against their Python path: the same bytes and bits for
 arguments that only the latter takes, the same refusals, the current stream."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 from horizon_kernels_b200 import _lib
+from horizon_kernels_b200 import backend as BE
 from horizon_kernels_b200 import kernels as K
 from horizon_kernels_b200 import layout as Lt
 
@@ -104,3 +107,67 @@ def test_the_current_stream_is_used():
         _decode(s, out)
     side.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("order", ["heads", "positions"])
+@pytest.mark.parametrize("opt", ["", "HAD", "K8"])
+@pytest.mark.parametrize("flat_rows", [True, False])
+def test_layer_calls_give_the_same(monkeypatch, order, opt, flat_rows):
+    """the backend's cache update and decode on the engine's own tensors, (tokens, heads * D) or (tokens, heads, D), new keys
+    and values as slices of one projection, fewer step tokens than rows: the same bytes and bits as through views and the
+    wrappers; what has another form is left to those, which serve or refuse it"""
+    if opt == "K8" and order == "positions":
+        pytest.skip("the K8V4 decode takes head-major pages only")
+    for name in ("HAD", "K8"):
+        monkeypatch.setenv(f"HORIZON_KVFP4_{name}", "1" if name == opt else "0")
+    D, k8 = 256 if opt == "K8" else 128, opt == "K8"
+    impl = BE.HorizonFp4Impl(KVH * G, D, D ** -0.5, num_kv_heads=KVH, kv_cache_dtype="nvfp4", max_num_seqs=8)
+    layer = SimpleNamespace(_k_scale_float=0.01, _v_scale_float=0.02)
+    slot, heads = (Lt.k8_slot_bytes(D), KVH) if k8 else (Lt.slot_bytes(D), 2 * KVH)
+    shape = (24, heads, PS, slot) if order == "heads" else (24, PS, heads, slot)
+    n = 200
+    kv = torch.randn(n, 2 * KVH * D, device="cuda").to(torch.bfloat16)
+    k, v = kv[:, :KVH * D], kv[:, KVH * D:]
+    q = torch.randn(B + 2, KVH * G * D, device="cuda").to(torch.bfloat16)
+    if not flat_rows:
+        k, v, q = k.view(n, KVH, D), v.view(n, KVH, D), q.view(B + 2, KVH * G, D)
+    slots = torch.randperm(24 * PS, device="cuda")[:n - 3]
+    meta = SimpleNamespace(num_reqs=B, num_actual_tokens=B, has_decode=True, prefill_rows=[], qlmax=1,
+                           block_table=torch.arange(24, dtype=torch.int32, device="cuda").view(B, 8),
+                           seq_lens=torch.tensor([100, 7, 128], dtype=torch.int32, device="cuda"),
+                           query_start_loc=torch.arange(B + 1, dtype=torch.int32, device="cuda"))
+    h, answers = _lib.host(), []
+
+    def logical(phys):
+        return phys if order == "heads" else phys.permute(0, 2, 1, 3)
+
+    def step(native):
+        def call(name):
+            def f(*a):
+                answers.append(getattr(h, name)(*a) if native else None)
+                return answers[-1]
+            return staticmethod(f)
+        monkeypatch.setattr(_lib, "_host", type("H", (), dict(
+            layer_write=call("layer_write"), layer_decode=call("layer_decode"), write=staticmethod(h.write),
+            decode=staticmethod(h.decode), prefill=staticmethod(h.prefill))))
+        phys, out = torch.zeros(shape, dtype=torch.uint8, device="cuda"), torch.zeros_like(q)
+        impl.do_kv_cache_update(layer, k, v, logical(phys), slots)
+        assert impl.forward(layer, q, k, v, logical(phys), meta, out) is out
+        return phys, out
+
+    want, got = step(False), step(True)
+    assert answers == [None, None, 0, 0]
+    assert torch.equal(want[0], got[0]) and want[0].any()
+    assert torch.equal(want[1], got[1]) and want[1][:B].any() and not want[1][B:].any()
+    cache = logical(got[0])
+    args = [k, v, cache, slots, impl._gk, impl._gv, D, True, None, k8]
+    wide = logical(torch.zeros(*shape[:3], 2 * slot, dtype=torch.uint8, device="cuda"))[..., ::2]
+    for i, bad in ((0, k.float()), (1, v[:-1]), (2, cache[:, 1:]), (2, wide), (3, slots.int()), (4, impl._gk[:1]), (6, 64),
+                   (8, impl._gk)):
+        assert h.layer_write(*args[:i], bad, *args[i + 1:]) is None
+    with pytest.raises(ValueError):
+        impl.do_kv_cache_update(layer, k, v, cache[:, 1:], slots)
+    with pytest.raises(TypeError):
+        impl.forward(layer, q.float(), k, v, cache, meta, torch.zeros_like(q))
+    with pytest.raises(ValueError):
+        impl.forward(layer, q, k, v, cache, meta, torch.zeros_like(q)[:1])
