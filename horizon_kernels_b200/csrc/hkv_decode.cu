@@ -7,8 +7,8 @@
 // the same (request, kv head) is a *piece*. A piece that covers its whole sequence is finished by the CTA and written
 // to the output; other pieces leave a normalised fp32 partial and a log2-sum-exp in the workspace. The log-sum-exp
 // combine of a split sequence runs inside the same launch: every CTA that wrote a piece of it draws a ticket from a
-// per-sequence counter when it is done, and the CTA that draws the last ticket merges all pieces in partition order
-// (fixed order => deterministic results, whoever merges). No CTA ever waits for another one.
+// counter when it is done, and the CTA that draws the last ticket merges all pieces in partition order
+// (fixed order => deterministic results, whoever merges); in two steps, by groups, when there are many. No CTA ever waits for another one.
 //
 // Inside a CTA, TG warps take the partition's units round-robin. Every warp owns a private ring of NS shared-memory
 // stages; it issues 1-D bulk copies (cp.async.bulk, completion on an mbarrier) for its own future units, driven by
@@ -35,6 +35,10 @@
 namespace hkv {
 
 constexpr int TG = 4;            // consumer warps per CTA
+// Fewest stream slots of a partition: two units per warp. A launch with little work then uses fewer CTAs, whose pieces are
+// fewer to merge: one request of 1024 (6453) tokens, 8 kv heads x 128, 10.3 us with 1, 9.5 with 4, 8.6 (11.7, 13.4 with 4) with 8;
+// 2000 tokens, 2 x 256, 18 / 14.7 / 14.0 us; four requests of 2048 tokens 11.3 / 11.4 / 11.5. Sixteen is slower for the short ones.
+constexpr int kMinPer = 8;
 constexpr bool kQueryPrefetch = true;   // ask for the next sequence's query rows (L2 prefetch) while a piece is computed
 constexpr int NTHREADS = TG * 32;
 constexpr int RPAD = 8;          // query rows per (request, kv head) of one pass, padded to the mma N tile
@@ -125,7 +129,7 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
   float* lbuf = mbuf + TG * RP;
   int* coarse = reinterpret_cast<int*>(smem + Sm::RING + Sm::BARS + Sm::MERGE);
   __shared__ SplitSeq split[2];
-  __shared__ int split_win[2];
+  __shared__ int split_win[2], group_win;
   unsigned pending = 0, drawn = 0;                  // bit 0 / 1: the partition's first / last piece belongs to a split
                                                     // sequence; .. and its ticket has been drawn already
 
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
   __syncthreads();
 
   const long long total = (long long)coarse[ngrp] * KVH;
-  const int per = (int)max(1ll, (total + n_parts - 1) / n_parts);
+  const int per = (int)max((long long)kMinPer, (total + n_parts - 1) / n_parts);
   const long long lo = (long long)part * per;
   const long long hi = min(total, lo + per);
   if (lo >= hi) {                                   // an idle partition
@@ -400,15 +404,10 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
   while (f_n < NS && (int)f_n < n_my) fetch_one(bars_a + 8 * f_n, ring_a + f_n * Gm::STAGE);
 
   // one thread, after a CTA barrier behind which every thread has fenced its share of the partial: counts this piece
-  // as finished; true when it was the sequence's last outstanding one (then the counter goes back to zero: every piece
-  // has arrived, nobody touches it again in this launch)
+  // as finished; true when it was the last outstanding one of its group (of its sequence, when that has few pieces)
   auto draw_ticket = [&](const SplitSeq& sq) -> int {
     const long long seq_u0 = sq.seq0 + PC;
-    const int first = (int)(seq_u0 / per), last = (int)((seq_u0 + sq.U - 1) / per);
-    __threadfence();
-    const int win = atomicAdd(tickets + last, 1) == last - first;
-    if (win) tickets[last] = 0;
-    return win;
+    return draw_piece(tickets, group_of(part, (int)(seq_u0 / per), (int)((seq_u0 + sq.U - 1) / per)));
   };
 
   // ---- compute side: walk the pieces of the partition
@@ -918,11 +917,28 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       const SplitSeq sq = split[i];
       const long long seq_u0 = sq.seq0 + PC;
       const int first = (int)(seq_u0 / per), last = (int)((seq_u0 + sq.U - 1) / per);
-      const int first_slot = (long long)first * per >= sq.seq0 ? 0 : 1;
-      for (int rb = 0; rb < sq.R; rb += RPAD)
-        merge_split<D, RP, NTHREADS, RPAD>(lse_ws, opart_ws, first, last, first_slot, sq.R, p.row0, p.G,
-                                          p.out + ((long long)sq.q0 * (KVH * p.G) + sq.h * p.G) * D,
-                                          (long long)KVH * p.G * D, p.v_scale, rb);
+      const int first_slot = 2 * first + ((long long)first * per >= sq.seq0 ? 0 : 1);
+      const Group gr = group_of(part, first, last);
+      MergeOut o{p.out + ((long long)sq.q0 * (KVH * p.G) + sq.h * p.G) * D, (long long)KVH * p.G * D, p.v_scale, p.row0, p.G, nullptr, nullptr};
+      Pieces pc{lse_ws, opart_ws, first_slot, first, 1, last - first + 1};
+      if (last - first + 1 > kGroupFrom) {
+        // the group's pieces into the partial of its first one; then, if that was the last group, the groups
+        const int slot0 = gr.first == first ? first_slot : 2 * gr.first;
+        MergeOut og = o;
+        og.row0 = nullptr;
+        og.part = opart_ws + (size_t)slot0 * RP * D;
+        og.lse = lse_ws + slot0 * RP;
+        merge_pieces<D, RP, NTHREADS>(Pieces{lse_ws, opart_ws, slot0, gr.first, 1, gr.last - gr.first + 1}, sq.R, og, obuf, Sm::MERGE / 4 - RP);
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) group_win = draw_group(tickets, first, last);
+        __syncthreads();
+        if (!group_win) continue;
+        __threadfence();
+        pc.step = kGroup;
+        pc.n = (last - first) / kGroup + 1;
+      }
+      merge_pieces<D, RP, NTHREADS>(pc, sq.R, o, obuf, Sm::MERGE / 4 - RP);
     }
   }
 

@@ -61,67 +61,176 @@ struct SplitSeq {
 };
 
 // ------------------------------------------------------------------------------------------------------- combine
-// Log-sum-exp merge of the pieces of one split sequence, run by the whole CTA that drew the sequence's last ticket.
-// The pieces live in slot `first_slot` of partition `first`, and in slot 0 of every later partition up to `last`.
-// w_i = 2^(lse_i - max) / sum, accumulated in partition order with a running maximum, so the result does not depend
-// on which CTA merges. out_row points at row 0 of the (request, kv head) group's first query token; rows of the next
-// token are tok_stride elements further. (Reference: hz4::combine_rg, kv_fp4_serving.py:518-558.)
-// RP: rows of a partial slot in the workspace; NT: threads of the calling group; the call merges rows rbase .. rbase + RB - 1
-template <int D, int RP, int NT, int RB = RP>
-__device__ __forceinline__ void merge_split(const float* lse_ws, const float* opart_ws, int first, int last,
-                                            int first_slot, int R, int row0, int G, __nv_bfloat16* out_row,
-                                            long long tok_stride, float v_scale, int rbase = 0) {
-  constexpr int IT = RB * (D / 2) / NT;      // (row, channel pair) items per thread
-  constexpr int GRP = 4;                             // pieces per round: GRP * IT independent loads in flight
+// Log-sum-exp merge of P pieces of one split sequence by the whole CTA (NT threads) that drew their last ticket: all pieces
+// of the sequence, or a group of them (kGroup below). w_i = 2^(lse_i - max), result sum w_i part_i / sum w_i, accumulated in partition
+// order, so it does not depend on which CTA merges. (Reference: hz4::combine_rg, kv_fp4_serving.py:518-558.)
+//
+// What bounds it is the latency of its loads from L2: nobody else works on the sequence by then. Up to eight pieces are loaded with
+// their log-sum-exps in one round trip. For more, the weights of all pieces come first, in one round trip through shared
+// memory, and a thread then has sixteen partials in flight whatever they weigh. Decode launch, before (rounds of four pieces under a
+// running maximum) -> now, with the two steps below: one request of 6453 tokens, 8 kv heads x 128, 55 pieces a head,
+// 22.1 -> 11.7 us (13.4 without kMinPer); of 32768 tokens, 2 x 256, 148 pieces, 98 -> 24; eight of 131072, 7 pieces, 220 -> 219.
+struct Pieces {
+  const float* lse;                                  // [slot][RP]
+  const float* part;                                 // [slot][RP][D]
+  int first_slot, first, step, n;                    // piece 0 lies in first_slot, piece i in slot 0 of partition first + i * step
+  __device__ __forceinline__ int slot(int i) const { return i == 0 ? first_slot : 2 * (first + i * step); }
+};
+// where the merged rows go: the output (row 0 of the (request, kv head) group's first query token; rows of the next token are
+// tok_stride elements further), or back into the partial of the first piece, which only this CTA reads any more
+struct MergeOut {
+  __nv_bfloat16* row0;                               // null: to `part` and `lse`
+  long long tok_stride;
+  float v_scale;
+  int first_row, G;                                  // row r of the pass is row first_row + r of the group
+  float* part;
+  float* lse;
+};
+template <int D>
+__device__ __forceinline__ void merge_store(const MergeOut& o, int row, int ch, float4 a, float total) {
+  const float inv = total > 0.0f ? (o.row0 ? o.v_scale : 1.0f) / total : 0.0f;
+  a.x *= inv; a.y *= inv; a.z *= inv; a.w *= inv;
+  if (o.row0) {
+    const int t = (o.first_row + row) / o.G, gq = o.first_row + row - t * o.G;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+    *reinterpret_cast<uint2*>(o.row0 + t * o.tok_stride + (long long)gq * D + ch) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  } else {
+    *reinterpret_cast<float4*>(o.part + (size_t)row * D + ch) = a;
+  }
+}
+// sm: RP + cap floats of shared memory
+template <int D, int RP, int NT>
+__device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const MergeOut& o, float* sm, int cap) {
+  constexpr int C4 = D / 4;                          // threads of a row, four channels each
+  constexpr int FEW = 8, GRP = 16;
   const float ninf = -__int_as_float(0x7f800000);
-  float mx[IT], tot[IT], n0[IT], n1[IT];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int P = pc.n, lane = threadIdx.x & 31;
+  auto fma4 = [](float4& a, const float4& v, float w) {
+    a.x = fmaf(v.x, w, a.x);
+    a.y = fmaf(v.y, w, a.y);
+    a.z = fmaf(v.z, w, a.z);
+    a.w = fmaf(v.w, w, a.w);
+  };
+  auto load = [&](int i, int row, int ch) {
+    return __ldcg(reinterpret_cast<const float4*>(pc.part + ((size_t)pc.slot(i) * RP + row) * D + ch));
+  };
+  if (P <= FEW && o.row0) {
+    constexpr int IT = 2, RB = IT * NT / C4;         // items of a thread, rows at a time
+    for (int rb = 0; rb < R; rb += RB) {
+      float ls[IT][FEW];
+      float4 v[IT][FEW];
 #pragma unroll
-  for (int it = 0; it < IT; ++it) { mx[it] = ninf; tot[it] = n0[it] = n1[it] = 0.0f; }
-  for (int pc0 = first; pc0 <= last; pc0 += GRP) {
-    float ls[IT][GRP];
-    float2 v[IT][GRP];
+      for (int it = 0; it < IT; ++it) {
+        const int idx = threadIdx.x + it * NT, row = rb + idx / C4, ch = idx % C4 * 4;
 #pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int idx = threadIdx.x + it * NT, row = rbase + idx / (D / 2), ch = (idx - (row - rbase) * (D / 2)) * 2;
+        for (int i = 0; i < FEW; ++i) {
+          const bool on = i < P && row < R;
+          ls[it][i] = on ? __ldcg(pc.lse + pc.slot(i) * RP + row) : ninf;
+          v[it][i] = on ? load(i, row, ch) : zero;
+        }
+      }
 #pragma unroll
-      for (int i = 0; i < GRP; ++i) {
-        const int pc = pc0 + i;
-        const int slot = pc * 2 + (pc == first ? first_slot : 0);
-        const bool on = pc <= last && row < R;
-        ls[it][i] = on ? __ldcg(lse_ws + slot * RP + row) : ninf;
-        v[it][i] = on ? __ldcg(reinterpret_cast<const float2*>(opart_ws + ((size_t)slot * RP + row) * D + ch))
-                      : make_float2(0.f, 0.f);
+      for (int it = 0; it < IT; ++it) {
+        const int idx = threadIdx.x + it * NT, row = rb + idx / C4, ch = idx % C4 * 4;
+        if (row >= R) continue;
+        float m = ls[it][0], tot = 0.0f;
+#pragma unroll
+        for (int i = 1; i < FEW; ++i) m = fmaxf(m, ls[it][i]);
+        float4 a = zero;
+#pragma unroll
+        for (int i = 0; i < FEW; ++i) {
+          if (ls[it][i] == ninf) continue;           // an empty piece: its partial is garbage and must not be used
+          const float w = exp2f(ls[it][i] - m);
+          tot += w;
+          fma4(a, v[it][i], w);
+        }
+        merge_store<D>(o, row, ch, a, tot);
       }
     }
+    return;
+  }
+  const int fit = max(1, min(R, cap / P));           // rows whose weights fit the shared memory
+  float* const sum = sm;
+  float* const wt = sm + RP;                         // [row][piece]
+  for (int rb = 0; rb < R; rb += fit) {
+    const int nr = min(fit, R - rb);
+    __syncthreads();                                 // the shared memory's last use is over
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr * P; i += NT) {
+      const int k = i / nr, r = i - k * nr;
+      wt[r * P + k] = __ldcg(pc.lse + pc.slot(k) * RP + rb + r);
+    }
+    __syncthreads();
+    for (int r = threadIdx.x >> 5; r < nr; r += NT / 32) {
+      float m = ninf, s = 0.0f;
+      for (int k = lane; k < P; k += 32) m = fmaxf(m, wt[r * P + k]);
 #pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      float gm = ls[it][0];
+      for (int x = 16; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+      for (int k = lane; k < P; k += 32) {
+        const float x = wt[r * P + k], w = x == ninf ? 0.0f : exp2f(x - m);
+        wt[r * P + k] = w;
+        s += w;
+      }
 #pragma unroll
-      for (int i = 1; i < GRP; ++i) gm = fmaxf(gm, ls[it][i]);
-      if (gm == ninf) continue;                      // only empty pieces in this round
-      const float nm = fmaxf(mx[it], gm);
-      const float keep = mx[it] == ninf ? 0.0f : exp2f(mx[it] - nm);
-      tot[it] *= keep; n0[it] *= keep; n1[it] *= keep;
-      mx[it] = nm;
-#pragma unroll
-      for (int i = 0; i < GRP; ++i) {
-        if (ls[it][i] == ninf) continue;             // an empty piece: its partial is garbage and must not be used
-        const float wgt = exp2f(ls[it][i] - nm);
-        tot[it] += wgt;
-        n0[it] += v[it][i].x * wgt;
-        n1[it] += v[it][i].y * wgt;
+      for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+      if (lane == 0) {
+        sum[r] = s;
+        if (!o.row0) o.lse[rb + r] = s > 0.0f ? m + log2f(s) : ninf;
       }
     }
-  }
+    __syncthreads();
+    for (int item = threadIdx.x; item < nr * C4; item += NT) {
+      const int r = item / C4, ch = item % C4 * 4;
+      const float* w = wt + r * P;
+      float4 a = zero;
+      for (int k0 = 0; k0 < P; k0 += GRP) {
+        float4 v[GRP];
+        float wg[GRP];
 #pragma unroll
-  for (int it = 0; it < IT; ++it) {
-    const int idx = threadIdx.x + it * NT, row = rbase + idx / (D / 2), ch = (idx - (row - rbase) * (D / 2)) * 2;
-    if (row >= R) continue;
-    const float inv = tot[it] > 0.0f ? v_scale / tot[it] : 0.0f;
-    const int t = (row0 + row) / G, gq = row0 + row - t * G;
-    *reinterpret_cast<__nv_bfloat162*>(out_row + t * tok_stride + (long long)gq * D + ch) =
-        __floats2bfloat162_rn(n0[it] * inv, n1[it] * inv);
+        for (int i = 0; i < GRP; ++i) {              // (an empty piece's partial is garbage and must not be used)
+          wg[i] = k0 + i < P ? w[k0 + i] : 0.0f;
+          v[i] = wg[i] > 0.0f ? load(k0 + i, rb + r, ch) : zero;
+        }
+#pragma unroll
+        for (int i = 0; i < GRP; ++i) fma4(a, v[i], wg[i]);
+      }
+      merge_store<D>(o, rb + r, ch, a, sum[r]);
+    }
   }
+}
+
+// Tickets. A sequence in more than kGroupFrom pieces is merged in two steps: groups of kGroup neighbouring pieces by the CTA
+// that finishes the group's last piece, then the groups by the CTA that merges the last of them. One CTA alone reads 150 pieces at
+// what one SM gets from L2 (the launch above with 148 pieces: 42 us), the groups are read by as many SMs (24 us). The line: 55
+// pieces take the same either way, 37 pieces 23.4 us in one step and 21.9 in two; 27 pieces 11.7 and 13.2. The counters lie in tickets[last partition of the group /
+// of the sequence]: finished pieces of a group in the low 16 bits, merged groups of the sequence in the high ones. They
+// are zero between launches. (No other split sequence ends in such a partition, so no other one counts there.)
+constexpr int kGroup = 16, kGroupFrom = 32;
+struct Group {
+  int first, last;                                   // partitions
+};
+__device__ __forceinline__ Group group_of(int part, int first, int last) {
+  if (last - first + 1 <= kGroupFrom) return {first, last};
+  const int g0 = first + (part - first) / kGroup * kGroup;
+  return {g0, min(g0 + kGroup - 1, last)};
+}
+// counts a finished piece of its group; true for the last one
+__device__ __forceinline__ bool draw_piece(int* tickets, Group g) {
+  __threadfence();
+  const int n = g.last - g.first + 1;
+  const bool win = (atomicAdd(tickets + g.last, 1) & 0xffff) == n - 1;
+  if (win) atomicSub(tickets + g.last, n);
+  return win;
+}
+// counts a merged group of the sequence; true for the last one
+__device__ __forceinline__ bool draw_group(int* tickets, int first, int last) {
+  __threadfence();
+  const int n = (last - first) / kGroup + 1;
+  const bool win = (atomicAdd(tickets + last, 0x10000) >> 16) == n - 1;
+  if (win) atomicSub(tickets + last, n << 16);
+  return win;
 }
 
 }  // namespace hkv

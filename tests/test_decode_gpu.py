@@ -397,3 +397,40 @@ def test_sixteen_rows_per_pass(KVH, G, ql, D):
         assert small.numel() < K.workspace_bytes(len(lens), KVH, G, D, ql)
         eight, _ = gpu_decode(c, qlmax=ql, ws=small)
         assert_close(eight, ref, "eight rows per pass")
+
+
+def _pieces_len(P):
+    """context length of a lone sequence in P pieces of eight stream slots (12 cost slots, then units of 32 tokens)"""
+    return 32 * (8 * P - 8) - 5
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("G,P", [(4, 2), (4, 8), (4, 9), (8, 16), (3, 17), (8, 32), (4, 33), (16, 33), (8, 48), (1, 49), (9, 49), (8, 65),
+                                 (16, 120)])
+def test_merge_in_one_and_two_steps(G, P, D):
+    """one sequence in P pieces: the direct merge (up to 8), the one through shared memory, groups of 16 from 33 on, whose last one
+    has 1, 16 or some pieces; G 16 and 9: the sixteen-row kernel. The counters are zero again afterwards, so a second call
+    on the workspace gives the same bits"""
+    c = build_decode_case(4100 + P, [_pieces_len(P)], 1, G, D, 16)
+    ref = oracle_decode(c)
+    out, ws = gpu_decode(c)
+    assert K.workspace_status(ws) == 0
+    assert_close(out, ref, f"{P} pieces")
+    assert not ws[256:256 + 4 * 4096].any()
+    again, _ = gpu_decode(c, ws=ws)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("D,kind", [(128, "hnd"), (256, "hnd"), (256, "nhd")])
+def test_groups_of_neighbouring_sequences(D, kind):
+    """several sequences with grouped merges beside short ones, whose pieces share partitions with them (a first piece in slot 1), at
+    two query tokens"""
+    lens = [40, _pieces_len(38), 3, _pieces_len(35), 700]
+    c = build_decode_case(4200, lens, 1, 4, D, 16, kind=kind, ql_list=[2] * len(lens))
+    ref = oracle_decode(c)
+    out, ws = gpu_decode(c, qlmax=2)
+    assert K.workspace_status(ws) == 0
+    assert_close(out, ref, "groups")
+    assert not ws[256:256 + 4 * 4096].any()
+    again, _ = gpu_decode(c, qlmax=2, ws=ws)
+    assert torch.equal(out, again)
