@@ -1159,7 +1159,7 @@ extern "C" int hkv_decode_k8(const void* q, const void* kd, const void* vd, cons
 extern "C" int hkv_combine(const void* workspace, size_t workspace_bytes, const int32_t* query_start_loc, int B,
                            int KVH, int G, int D, int qlmax, float v_scale, void* out, void* stream) {
   using namespace hkv;
-  // The log-sum-exp combine runs inside the decode launch (merge_split above): when hkv_decode's kernels have finished,
+  // The log-sum-exp combine runs inside the decode launch (merge_pieces): when hkv_decode's kernels have finished,
   // `out` is complete. This entry point is kept so that callers written against the three-call sequence of the
   // reference (write, decode, combine) keep working; it checks its arguments like before and launches nothing.
   (void)v_scale; (void)stream;

@@ -69,7 +69,7 @@ struct SplitSeq {
 // their log-sum-exps in one round trip. For more, the weights of all pieces come first, in one round trip through shared
 // memory, and a thread then has sixteen partials in flight whatever they weigh. Decode launch, before (rounds of four pieces under a
 // running maximum) -> now, with the two steps below: one request of 6453 tokens, 8 kv heads x 128, 55 pieces a head,
-// 22.1 -> 11.7 us (13.4 without kMinPer); of 32768 tokens, 2 x 256, 148 pieces, 98 -> 24; eight of 131072, 7 pieces, 220 -> 219.
+// 22.1 -> 11.7 us (13.6 without kMinPer); of 32768 tokens, 2 x 256, 148 pieces, 98 -> 24; eight of 131072, 7 pieces, 220 -> 219.
 struct Pieces {
   const float* lse;                                  // [slot][RP]
   const float* part;                                 // [slot][RP][D]
@@ -203,8 +203,8 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
 
 // Tickets. A sequence in more than kGroupFrom pieces is merged in two steps: groups of kGroup neighbouring pieces by the CTA
 // that finishes the group's last piece, then the groups by the CTA that merges the last of them. One CTA alone reads 150 pieces at
-// what one SM gets from L2 (the launch above with 148 pieces: 42 us), the groups are read by as many SMs (24 us). The line: 55
-// pieces take the same either way, 37 pieces 23.4 us in one step and 21.9 in two; 27 pieces 11.7 and 13.2. The counters lie in tickets[last partition of the group /
+// what one SM gets from L2 (the launch above with 148 pieces: 42 us), the groups are read by as many SMs (24 us). The line:
+// 33 pieces at head_dim 256 took 23.4 us in one step and 21.3 in two, 26 at head_dim 128 11.7 and 13.2. The counters lie in tickets[last partition of the group /
 // of the sequence]: finished pieces of a group in the low 16 bits, merged groups of the sequence in the high ones. They
 // are zero between launches. (No other split sequence ends in such a partition, so no other one counts there.)
 constexpr int kGroup = 16, kGroupFrom = 32;
