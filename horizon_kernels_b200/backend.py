@@ -303,6 +303,8 @@ def _build_classes():
             """reference backend.py:389-403"""
             gk, gv = (self._gk, self._gv) if self._gk is not None else self._scales(layer, key.device)
             D = self.head_size
+            if self._views is None:                   # so that the layer's first prefill does not wait for them
+                self._cache_views(kv_cache)
             # the usual arguments are taken as they are; through the views below the call takes half as long again
             rc = (_lib._host or _lib.host()).layer_write(key, value, kv_cache, slot_mapping, gk, gv, D, self.search,
                                                          self._rot(key.device) if self.had else None, self.k8)
