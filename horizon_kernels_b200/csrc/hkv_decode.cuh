@@ -153,7 +153,7 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
   }
   const int fit = max(1, min(R, cap / P));           // rows whose weights fit the shared memory
   float* const sum = sm;
-  float* const wt = sm + RP;                         // [row][piece]
+  float* const wt = sm + RP;                         // [row][piece]; -0: an empty piece, whose partial is garbage and must not be used
   for (int rb = 0; rb < R; rb += fit) {
     const int nr = min(fit, R - rb);
     __syncthreads();                                 // the shared memory's last use is over
@@ -169,7 +169,7 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
 #pragma unroll
       for (int x = 16; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
       for (int k = lane; k < P; k += 32) {
-        const float x = wt[r * P + k], w = x == ninf ? 0.0f : exp2f(x - m);
+        const float x = wt[r * P + k], w = x == ninf ? -0.0f : exp2f(x - m);
         wt[r * P + k] = w;
         s += w;
       }
@@ -189,9 +189,9 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
         float4 v[GRP];
         float wg[GRP];
 #pragma unroll
-        for (int i = 0; i < GRP; ++i) {              // (an empty piece's partial is garbage and must not be used)
-          wg[i] = k0 + i < P ? w[k0 + i] : 0.0f;
-          v[i] = wg[i] > 0.0f ? load(k0 + i, rb + r, ch) : zero;
+        for (int i = 0; i < GRP; ++i) {              // (a weight that underflowed to zero still carries a NaN or an infinity)
+          wg[i] = k0 + i < P ? w[k0 + i] : -0.0f;
+          v[i] = __float_as_int(wg[i]) >= 0 ? load(k0 + i, rb + r, ch) : zero;
         }
 #pragma unroll
         for (int i = 0; i < GRP; ++i) fma4(a, v[i], wg[i]);

@@ -434,3 +434,25 @@ def test_groups_of_neighbouring_sequences(D, kind):
     assert not ws[256:256 + 4 * 4096].any()
     again, _ = gpu_decode(c, qlmax=2, ws=ws)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("D,G", [(128, 4), (256, 8), (256, 16)])
+@pytest.mark.parametrize("P,first,last", [(3, 1, 1), (20, 3, 3), (40, 5, 5), (40, 16, 31)])
+def test_a_nan_under_no_weight_is_kept(P, first, last, D, G):
+    """a NaN value scale in a piece (of a group, or of a whole group of sixteen) whose weight underflows to zero in the merge:
+    0 * NaN is NaN however many pieces there are; the other channels are those of the other pieces"""
+    L = _pieces_len(P)
+    c = build_decode_case(4300 + P, [L], 1, G, D, 16, gscale=(1.0, 0.5))
+    t0, t1 = 32 * max(0, 8 * first - 4), 32 * (8 * last + 4)             # the tokens of the pieces first .. last
+    c["key"][:], c["q"][:] = 0x4100, 0x3F80                              # keys of 8, of -8 in those pieces, queries of 1:
+    c["key"][t0:t1] = 0xC100                                             # scores 260 apart (base 2) and more
+    dev = c["cache"].phys.device
+    K.write(bf16_tensor(c["key"]), bf16_tensor(c["val"]), c["cache"].flat, c["cache"].strides, 16,
+            torch.from_numpy(c["slots"]).to(dev), torch.from_numpy(c["gk"]).to(dev), torch.from_numpy(c["gv"]).to(dev))
+    ref = oracle_decode(c)
+    slot = int(c["slots"][t0 + 40])
+    c["cache"].phys[slot // 16, 1, slot % 16, D // 2] = 0x7F             # scale of the value's channels 0 .. 15
+    out, ws = gpu_decode(c)
+    assert K.workspace_status(ws) == 0
+    assert torch.isnan(out[..., :16]).all()
+    assert_close(out[..., 16:], ref[..., 16:], f"{P} pieces")
