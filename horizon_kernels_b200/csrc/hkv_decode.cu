@@ -97,7 +97,7 @@ struct Geo {
 // QT: 8-row query tiles of one pass (1, or 2: sixteen query rows per kv head read the cache once). At head_dim 256 the two
 // tiles' accumulators take 128 registers: the query fragments lie in shared memory (QSM), where a piece's merge buffer lies
 // afterwards, a unit's two 16-token blocks are worked on one after the other and the merge takes one tile at a time, so that
-// two CTAs still fit an SM (245 registers, none spilled). 96 requests of 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query
+// two CTAs still fit an SM (251 registers, none spilled). 96 requests of 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query
 // tokens, rotated keys: 102 us in one pass against 146 in two of eight rows. (At head_dim 128 the fragments stay in registers:
 // the same layout there lets a third CTA in, and took 62 to 67 us where this one takes 59.)
 template <int D, int LAYOUT, int QT = 1>

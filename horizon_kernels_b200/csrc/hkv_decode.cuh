@@ -65,8 +65,8 @@ struct SplitSeq {
 // of the sequence, or a group of them (kGroup below). w_i = 2^(lse_i - max), result sum w_i part_i / sum w_i, accumulated in partition
 // order, so it does not depend on which CTA merges. (Reference: hz4::combine_rg, kv_fp4_serving.py:518-558.)
 //
-// What bounds it is the latency of its loads from L2: nobody else works on the sequence by then. Up to eight pieces are loaded with
-// their log-sum-exps in one round trip. For more, the weights of all pieces come first, in one round trip through shared
+// What bounds it is the latency of its loads from L2: nobody else works on the sequence by then. Up to eight pieces (FEW) are loaded with
+// their log-sum-exps in one round trip per eight rows (four at head_dim 256). For more, the weights of all pieces come first, in one round trip through shared
 // memory, and a thread then has sixteen partials in flight whatever they weigh. Decode launch, before (rounds of four pieces under a
 // running maximum) -> now, with the two steps below: one request of 6453 tokens, 8 kv heads x 128, 55 pieces a head,
 // 22.1 -> 11.7 us (13.6 without kMinPer); of 32768 tokens, 2 x 256, 148 pieces, 98 -> 24; eight of 131072, 7 pieces, 220 -> 219.
@@ -103,7 +103,9 @@ __device__ __forceinline__ void merge_store(const MergeOut& o, int row, int ch, 
 template <int D, int RP, int NT>
 __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const MergeOut& o, float* sm, int cap) {
   constexpr int C4 = D / 4;                          // threads of a row, four channels each
-  constexpr int FEW = 8, GRP = 16;
+  // (six in the sixteen-row kernel at head_dim 256, whose registers are the tightest: with eight it takes 255 and spills. 96 requests of
+  // 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query tokens: 96.6 us with eight, 93.9 with six, 97.9 with four)
+  constexpr int FEW = D == 256 && RP == 16 ? 6 : 8, GRP = 16;
   const float ninf = -__int_as_float(0x7f800000);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const int P = pc.n, lane = threadIdx.x & 31;
