@@ -279,6 +279,14 @@ def _build_classes():
             self._views = (kv_cache.data_ptr(), tuple(kv_cache.stride()), out)
             return out
 
+        def _keep_to(self, kv_cache):
+            """the views are those of this cache's memory, also where the native side takes the call without them: they hold the
+            storage, so those of a cache that the engine has replaced would keep it alive (and the layer's first prefill does not
+            wait for them)"""
+            v = self._views
+            if v is None or v[0] != kv_cache.data_ptr():
+                self._cache_views(kv_cache)
+
         def _scales(self, layer, device):
             if self._gk is None:
                 self._gk = torch.full((self.num_kv_heads,), float(layer._k_scale_float), device=device)
@@ -303,8 +311,7 @@ def _build_classes():
             """reference backend.py:389-403"""
             gk, gv = (self._gk, self._gv) if self._gk is not None else self._scales(layer, key.device)
             D = self.head_size
-            if self._views is None:                   # so that the layer's first prefill does not wait for them
-                self._cache_views(kv_cache)
+            self._keep_to(kv_cache)
             # the usual arguments are taken as they are; through the views below the call takes half as long again
             rc = (_lib._host or _lib.host()).layer_write(key, value, kv_cache, slot_mapping, gk, gv, D, self.search,
                                                          self._rot(key.device) if self.had else None, self.k8)
@@ -331,6 +338,7 @@ def _build_classes():
             st = self._state(query.device)
             gk, gv = (self._gk, self._gv) if self._gk is not None else self._scales(layer, query.device)
             decode = m.has_decode and m.num_reqs > 0
+            self._keep_to(kv_cache)
             if decode:                                # as in do_kv_cache_update: the usual arguments as they are
                 rc = (_lib._host or _lib.host()).layer_decode(
                     query, kv_cache, m.block_table, m.seq_lens, m.query_start_loc, T, self.scale, float(layer._v_scale_float),

@@ -106,3 +106,38 @@ def test_register_is_gated(monkeypatch):
     import horizon_kernels_b200
     monkeypatch.delenv("HORIZON_KVFP4", raising=False)
     horizon_kernels_b200.register()                       # does nothing, imports nothing
+
+
+@pytest.mark.parametrize("call", ["update", "forward"])
+def test_a_replaced_cache_is_let_go(monkeypatch, call):
+    """an engine that replaces its cache (sleep and wake, a resized pool): the layer's first call on the new one drops what it holds of the
+    old one, also where the native side serves the call without the views"""
+    import gc
+    import weakref
+
+    import numpy as np
+
+    from horizon_kernels_b200 import _lib
+    monkeypatch.setattr(_lib, "_host", SimpleNamespace(layer_write=lambda *a: 0, layer_decode=lambda *a: 0))
+    impl = BE.HorizonFp4Impl(8, 128, 0.1, num_kv_heads=2, kv_cache_dtype="nvfp4")
+    impl._state = lambda device: {"ws": None}
+    layer = SimpleNamespace(_k_scale_float=1.0, _v_scale_float=1.0)
+    kv, q = torch.zeros(3, 2 * 128, dtype=torch.bfloat16), torch.zeros(3, 8 * 128, dtype=torch.bfloat16)
+    meta = SimpleNamespace(num_actual_tokens=3, has_decode=True, num_reqs=3, prefill_rows=[], block_table=None, seq_lens=None,
+                           query_start_loc=None, qlmax=1)
+
+    def cache():
+        mem = np.zeros((4, 4, 16, 72), np.uint8)
+        return torch.from_numpy(mem), weakref.ref(mem)
+
+    old, freed = cache()
+    impl.do_kv_cache_update(layer, kv, kv, old, torch.zeros(3, dtype=torch.int64))
+    assert impl._views is not None
+    new, _ = cache()
+    del old
+    if call == "update":
+        impl.do_kv_cache_update(layer, kv, kv, new, torch.zeros(3, dtype=torch.int64))
+    else:
+        impl.forward(layer, q, kv, kv, new, meta, q.clone())
+    gc.collect()
+    assert freed() is None
