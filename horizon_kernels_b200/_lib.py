@@ -105,14 +105,17 @@ class _NoHost:
 
 
 def load_host(path):
-    """the host module at `path`; raises where it is absent, does not load or was built for another torch (it is bound to the
-    binary interface of one torch version)"""
+    """the host module at `path`; raises where it is absent, does not load, was built for another torch (it is bound to the
+    binary interface of one torch version) or from a source that had fewer functions"""
     import torch
     spec = importlib.util.spec_from_file_location("hkv_host", path)
     h = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(h)
     if h.torch_version != str(torch.__version__):
         raise ImportError(f"built for torch {h.torch_version}, not {torch.__version__}")
+    missing = [n for n in (*vars(_NoHost), "bind") if not n.startswith("_") and not hasattr(h, n)]
+    if missing:
+        raise ImportError(f"built from an older source, without {', '.join(missing)}")
     return h
 
 
@@ -124,14 +127,14 @@ def host():
         L = load()
         try:
             h = load_host(HOST_PATH)
-        except (ImportError, OSError, AttributeError) as e:
+            h.bind(*[C.cast(f, C.c_void_p).value for f in (
+                L.hkv_write, L.hkv_write_rot, L.hkv_write_k8, L.hkv_decode, L.hkv_decode_rot, L.hkv_decode_k8,
+                L.hkv_prefill_scratch_bytes, L.hkv_prefill)])
+        except (ImportError, OSError, AttributeError, TypeError) as e:       # (TypeError: it binds another set of entry points)
             warnings.warn(f"{HOST_PATH} does not load, every call takes the slower Python path: {e} (rebuild it with "
                           "`python -m horizon_kernels_b200.build`)", RuntimeWarning, stacklevel=3)
             _host = _NoHost
             return _host
-        h.bind(*[C.cast(f, C.c_void_p).value for f in (
-            L.hkv_write, L.hkv_write_rot, L.hkv_write_k8, L.hkv_decode, L.hkv_decode_rot, L.hkv_decode_k8,
-            L.hkv_prefill_scratch_bytes, L.hkv_prefill)])
         _host = h
     return _host
 

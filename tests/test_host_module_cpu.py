@@ -60,3 +60,29 @@ def test_the_built_module_is_this_torch_s(unloaded, monkeypatch):
     with warnings.catch_warnings():
         warnings.simplefilter("error")
         assert _lib.host() is not _lib._NoHost
+
+
+@pytest.mark.parametrize("missing", [n for n in vars(_lib._NoHost) if not n.startswith("_")] + ["bind"])
+def test_a_module_of_an_older_source(unloaded, monkeypatch, tmp_path, missing):
+    """built for this torch, before the source gained a function (libraries are not under version control, so a checkout that is brought
+    up to date has one until the next build): the Python path serves, and the build replaces it"""
+    old = tmp_path / "hkv_host.py"                   # (the loader goes by the suffix)
+    names = [n for n in vars(_lib._NoHost) if not n.startswith("_")]
+    old.write_text(f"torch_version = {str(torch.__version__)!r}\n" + "".join(
+        f"def {n}(*a):\n    return None\n" for n in [*names, "bind"] if n != missing))
+    monkeypatch.setattr(_lib, "HOST_PATH", str(old))
+    with pytest.warns(RuntimeWarning, match="Python path") as w:
+        _calls()
+        assert _lib.host().layer_write() is None and _lib.host().layer_decode() is None
+    assert len(w) == 1
+    monkeypatch.setattr(build, "HOST", str(old))
+    assert not build._host_loads()
+
+
+def test_a_module_that_binds_other_entry_points(unloaded, monkeypatch, tmp_path):
+    old = tmp_path / "hkv_host.py"
+    old.write_text(f"torch_version = {str(torch.__version__)!r}\ndef bind(a, b):\n    pass\n" + "".join(
+        f"def {n}(*a):\n    return None\n" for n in vars(_lib._NoHost) if not n.startswith("_")))
+    monkeypatch.setattr(_lib, "HOST_PATH", str(old))
+    with pytest.warns(RuntimeWarning, match="Python path"):
+        _calls()
