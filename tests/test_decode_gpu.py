@@ -456,3 +456,32 @@ def test_a_nan_under_no_weight_is_kept(P, first, last, D, G):
     assert K.workspace_status(ws) == 0
     assert torch.isnan(out[..., :16]).all()
     assert_close(out[..., 16:], ref[..., 16:], f"{P} pieces")
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("G", [1, 2])
+@pytest.mark.parametrize("P", [2, 6, 7, 8, 9, 17, 32, 33, 40, 49, 65])
+def test_an_empty_row_in_the_last_piece(P, G, D):
+    """the last unit of a sequence in P pieces (one sequence per head, partitions of eight slots) is a piece of its own with three tokens:
+    of eight query tokens only the last three see it, the other rows' partials there must not count. Eight rows (G 1) and the
+    sixteen-row kernel (G 2); the direct merge (up to 8 pieces, 6 at 256 x 16 rows), the one through shared memory, groups of 16
+    whose last one is that single piece (33, 49, 65) or holds it (40). What the workspace holds besides its counters is NaN before"""
+    U = 8 * P - 11                                       # units; the 12 cost slots of the sequence come before them
+    first, last = 12 // 8, (12 + U - 1) // 8
+    assert last - first + 1 == P and (12 + U - 1) % 8 == 0
+    c = build_decode_case(4500 + P, [32 * (U - 1) + 3, 5], 1, G, D, 16, ql_list=[8, 8])
+    ref = oracle_decode(c)
+    q1 = int(c["qsl"][1])
+    ref[q1:q1 + 3] = 0.0                                 # context 5, eight query tokens: the first three see nothing at all
+    ws = K.alloc_workspace(2, 1, G, D, 8, c["cache"].phys.device)
+    ws[256 + 4 * 4096:] = 0xFF
+    out, _ = gpu_decode(c, qlmax=8, ws=ws)
+    assert K.workspace_status(ws) == 0
+    R = 8 * G                                            # rows of the pass, and of a slot of the log-sum-exps
+    lse = ws[256 + 4 * 4096:].view(torch.float32)[2 * last * R:(2 * last + 1) * R].cpu()
+    assert (lse[:5 * G] == -np.inf).all() and torch.isfinite(lse[5 * G:]).all()
+    assert_close(out, ref, f"{P} pieces")
+    assert (out[q1:q1 + 3] == 0).all()
+    assert not ws[256:256 + 4 * 4096].any()
+    again, _ = gpu_decode(c, qlmax=8, ws=ws)
+    assert torch.equal(out, again)
