@@ -14,12 +14,12 @@ namespace hkv {
 // Layout of the decode workspace (all offsets from the 256-byte aligned base):
 //   Header | tickets[kMaxParts] int | lse[n_parts][2][RPAD] fp32 | opart[n_parts][2][RPAD][D] fp32
 // Each decode partition (one CTA) owns two partial slots: slot 0 for a sequence piece that begins the partition,
-// slot 1 for a piece that ends it while the sequence continues in the next partition. tickets[p] counts, in its low half, the finished
-// pieces of the split sequence (of its group of pieces, when there are many) that ENDS in partition p, in its high half the merged
-// groups of that sequence; the CTA that completes a count merges and takes the count off again, so the counters are zero
-// between launches (the workspace starts zero-filled). The ticket
-// table has a fixed size and place, so that launches with different partition counts on one workspace (another batch
-// size or `splits` cap moves the partial slots) never write partials over a counter.
+// slot 1 for a piece that ends it while the sequence continues in the next partition. tickets[p] counts, in its low half, the
+// finished pieces of the split sequence (of its group of pieces, when there are many) that ENDS in partition p, in its high
+// half the merged groups of that sequence; the CTA that completes a count merges and takes the count off again, so the
+// counters are zero between launches (the workspace starts zero-filled). The ticket table has a fixed size and place, so that
+// launches with different partition counts on one workspace (another batch size or `splits` cap moves the partial slots)
+// never write partials over a counter.
 struct Header {
   int status;      // HKV_OK or HKV_ERR_DEVICE_WAIT, set by a kernel whose bounded wait ran out
   int pad[15];

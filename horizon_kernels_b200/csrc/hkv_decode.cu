@@ -8,7 +8,8 @@
 // to the output; other pieces leave a normalised fp32 partial and a log2-sum-exp in the workspace. The log-sum-exp
 // combine of a split sequence runs inside the same launch: every CTA that wrote a piece of it draws a ticket from a
 // counter when it is done, and the CTA that draws the last ticket merges all pieces in partition order
-// (fixed order => deterministic results, whoever merges); in two steps, by groups, when there are many. No CTA ever waits for another one.
+// (fixed order => deterministic results, whoever merges); in two steps, by groups, when there are many. No CTA ever waits for
+// another one.
 //
 // Inside a CTA, TG warps take the partition's units round-robin. Every warp owns a private ring of NS shared-memory
 // stages; it issues 1-D bulk copies (cp.async.bulk, completion on an mbarrier) for its own future units, driven by
@@ -36,8 +37,11 @@ namespace hkv {
 
 constexpr int TG = 4;            // consumer warps per CTA
 // Fewest stream slots of a partition: two units per warp. A launch with little work then uses fewer CTAs, whose pieces are
-// fewer to merge: one request of 1024 (6453) tokens, 8 kv heads x 128, 10.3 us with 1, 9.5 with 4, 8.6 (11.7, 13.4 with 4) with 8;
-// 2000 tokens, 2 x 256, 18 / 14.7 / 14.0 us; four requests of 2048 tokens 11.3 / 11.4 / 11.5. Sixteen is slower for the short ones.
+// fewer to merge. With 1 / 4 / 8 / 16, launches back to back: one request of 1024 tokens, 8 kv heads x 128, 12.9 / 10.9 / 11.4 /
+// 12.4 us, of 6453 15.9 / 15.9 / 14.7 / 14.3; of 2000, 2 x 256, 20.9 / 17.2 / 16.5 / 17.2; two of 1000 with two query tokens, 2 x
+// 256, 29.6 / 21.1 / 19.4 / 22.3; four of 2048, 8 x 128, 13.7 / 13.7 / 14.2 / 14.6. What it costs: 24 to 130 sequences of 200 to 450
+// tokens, which are few pieces anyway, get two units per warp where one would do (12 requests of 300 tokens, 4 x 256: 14.1 us
+// with 4, 15.1 with 8; positions outermost 15.9 and 18.9). One value for all layouts: the page orders give the same bits.
 constexpr int kMinPer = 8;
 constexpr bool kQueryPrefetch = true;   // ask for the next sequence's query rows (L2 prefetch) while a piece is computed
 constexpr int NTHREADS = TG * 32;
@@ -919,7 +923,8 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
       const int first = (int)(seq_u0 / per), last = (int)((seq_u0 + sq.U - 1) / per);
       const int first_slot = 2 * first + ((long long)first * per >= sq.seq0 ? 0 : 1);
       const Group gr = group_of(part, first, last);
-      MergeOut o{p.out + ((long long)sq.q0 * (KVH * p.G) + sq.h * p.G) * D, (long long)KVH * p.G * D, p.v_scale, p.row0, p.G, nullptr, nullptr};
+      MergeOut o{p.out + ((long long)sq.q0 * (KVH * p.G) + sq.h * p.G) * D, (long long)KVH * p.G * D, p.v_scale, p.row0, p.G,
+                 nullptr, nullptr};
       Pieces pc{lse_ws, opart_ws, first_slot, first, 1, last - first + 1};
       if (last - first + 1 > kGroupFrom) {
         // the group's pieces into the partial of its first one; then, if that was the last group, the groups
@@ -928,7 +933,8 @@ __global__ void __launch_bounds__(NTHREADS, QT == 2 ? 2 : Geo<D, LAYOUT>::MINB) 
         og.row0 = nullptr;
         og.part = opart_ws + (size_t)slot0 * RP * D;
         og.lse = lse_ws + slot0 * RP;
-        merge_pieces<D, RP, NTHREADS>(Pieces{lse_ws, opart_ws, slot0, gr.first, 1, gr.last - gr.first + 1}, sq.R, og, obuf, Sm::MERGE / 4 - RP);
+        merge_pieces<D, RP, NTHREADS>(Pieces{lse_ws, opart_ws, slot0, gr.first, 1, gr.last - gr.first + 1}, sq.R, og, obuf,
+                                      Sm::MERGE / 4 - RP);
         __threadfence();
         __syncthreads();
         if (tid == 0) group_win = draw_group(tickets, first, last);

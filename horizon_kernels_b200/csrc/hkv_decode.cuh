@@ -62,14 +62,16 @@ struct SplitSeq {
 
 // ------------------------------------------------------------------------------------------------------- combine
 // Log-sum-exp merge of P pieces of one split sequence by the whole CTA (NT threads) that drew their last ticket: all pieces
-// of the sequence, or a group of them (kGroup below). w_i = 2^(lse_i - max), result sum w_i part_i / sum w_i, accumulated in partition
-// order, so it does not depend on which CTA merges. (Reference: hz4::combine_rg, kv_fp4_serving.py:518-558.)
+// of the sequence, or a group of them (kGroup below). w_i = 2^(lse_i - max), result sum w_i part_i / sum w_i, accumulated in
+// partition order, so it does not depend on which CTA merges. (Reference: hz4::combine_rg, kv_fp4_serving.py:518-558.)
 //
-// What bounds it is the latency of its loads from L2: nobody else works on the sequence by then. Up to eight pieces (FEW) are loaded with
-// their log-sum-exps in one round trip per eight rows (four at head_dim 256). For more, the weights of all pieces come first, in one round trip through shared
-// memory, and a thread then has sixteen partials in flight whatever they weigh. Decode launch, before (rounds of four pieces under a
-// running maximum) -> now, with the two steps below: one request of 6453 tokens, 8 kv heads x 128, 55 pieces a head,
-// 22.1 -> 11.7 us (13.6 without kMinPer); of 32768 tokens, 2 x 256, 148 pieces, 98 -> 24; eight of 131072, 7 pieces, 220 -> 219.
+// What bounds it is the latency of its loads from L2: nobody else works on the sequence by then. Up to eight pieces (FEW) are
+// loaded with their log-sum-exps in one round trip per eight rows (four at head_dim 256). For more, the weights of all pieces
+// come first, in one round trip through shared memory, and a thread then has sixteen partials in flight whatever they weigh.
+// Launches back to back (`microbench decode --iters 2000 --batch B --min-len L --max-len L ..`), before (rounds of four pieces
+// under a running maximum, partitions of any size) -> now, with the two steps below and kMinPer: one request of 6453 tokens,
+// 8 kv heads x 128, 51 -> 26 pieces a head, 24.4 -> 14.7 us (15.9 with the 51 pieces); of 32768 tokens, 2 x 256, 147 -> 129
+// pieces, 101 -> 26.5; eight of 131072, 8 x 128, 7 pieces, 236 both.
 struct Pieces {
   const float* lse;                                  // [slot][RP]
   const float* part;                                 // [slot][RP][D]
@@ -103,8 +105,8 @@ __device__ __forceinline__ void merge_store(const MergeOut& o, int row, int ch, 
 template <int D, int RP, int NT>
 __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const MergeOut& o, float* sm, int cap) {
   constexpr int C4 = D / 4;                          // threads of a row, four channels each
-  // (six in the sixteen-row kernel at head_dim 256, whose registers are the tightest: with eight it takes 255 and spills. 96 requests of
-  // 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query tokens: 96.6 us with eight, 93.9 with six, 97.9 with four)
+  // (six in the sixteen-row kernel at head_dim 256, whose registers are the tightest: with eight it takes 255 and spills. 96
+  // requests of 0.5k to 16k tokens, 2 kv heads, group 8 x 2 query tokens: 96.6 us with eight, 93.9 with six, 97.9 with four)
   constexpr int FEW = D == 256 && RP == 16 ? 6 : 8, GRP = 16;
   const float ninf = -__int_as_float(0x7f800000);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -155,7 +157,7 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
   }
   const int fit = max(1, min(R, cap / P));           // rows whose weights fit the shared memory
   float* const sum = sm;
-  float* const wt = sm + RP;                         // [row][piece]; -0: an empty piece, whose partial is garbage and must not be used
+  float* const wt = sm + RP;                         // [row][piece]; -0: an empty piece, whose partial is garbage, not to be used
   for (int rb = 0; rb < R; rb += fit) {
     const int nr = min(fit, R - rb);
     __syncthreads();                                 // the shared memory's last use is over
@@ -204,11 +206,13 @@ __device__ __forceinline__ void merge_pieces(const Pieces& pc, int R, const Merg
 }
 
 // Tickets. A sequence in more than kGroupFrom pieces is merged in two steps: groups of kGroup neighbouring pieces by the CTA
-// that finishes the group's last piece, then the groups by the CTA that merges the last of them. One CTA alone reads 150 pieces at
-// what one SM gets from L2 (the launch above with 148 pieces: 42 us), the groups are read by as many SMs (24 us). The line:
-// 33 pieces at head_dim 256 took 23.4 us in one step and 21.3 in two, 26 at head_dim 128 11.7 and 13.2. The counters lie in tickets[last partition of the group /
-// of the sequence]: finished pieces of a group in the low 16 bits, merged groups of the sequence in the high ones. They
-// are zero between launches. (No other split sequence ends in such a partition, so no other one counts there.)
+// that finishes the group's last piece, then the groups by the CTA that merges the last of them. One CTA alone reads 129 pieces
+// at what one SM gets from L2 (the launch above: 40.9 us), the groups are read by as many SMs (26.5 us). The line, one request,
+// in one step / in two: 8 x 128, 26 pieces (6453 tokens) 14.7 / 16.7 us, 48 pieces 16.6 / 17.4, 54 pieces 21.3 / 21.6; 2 x 256,
+// 17 pieces 18.6 / 20.8, 31 pieces 20.3 / 21.4, 33 pieces 21.0 / 21.2, 48 pieces 23.2 / 22.0; sixteen rows there, 33 pieces
+// 31.4 / 29.6. The counters lie in tickets[last partition of the group / of the sequence]: finished pieces of a group in the low
+// 16 bits, merged groups of the sequence in the high ones. They are zero between launches. (No other split sequence ends in
+// such a partition, so no other one counts there.)
 constexpr int kGroup = 16, kGroupFrom = 32;
 struct Group {
   int first, last;                                   // partitions

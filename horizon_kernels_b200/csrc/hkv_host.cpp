@@ -1,7 +1,7 @@
-// Native side of kernels.write, kernels.decode_ragged and kernels.prefill, and of the backend's cache update and decode: takes the
-// callers' Python arguments as they are, checks them and calls the C ABI (include/hkv.h). What the wrappers do per call in Python (about forty attribute reads and checks, a
-// device context, the conversion of 25 ctypes arguments) costs 20 to 25 microseconds, longer than a small decode step runs
-// on the GPU; here it costs two.
+// Native side of kernels.write, kernels.decode_ragged and kernels.prefill, and of the backend's cache update and decode: takes
+// the callers' Python arguments as they are, checks them and calls the C ABI (include/hkv.h). What the wrappers do per call in
+// Python (about forty attribute reads and checks, a device context, the conversion of 25 ctypes arguments) costs 20 to 25
+// microseconds, longer than a small decode step runs on the GPU; here it costs two.
 //
 // Each function answers None when an argument is not of the plain form it knows (wrong type, shape or device, a tensor
 // subclass, anything that throws): nothing has been launched then, and the Python path checks, raises or serves the
